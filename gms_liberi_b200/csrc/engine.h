@@ -157,12 +157,19 @@ struct PlanHost {
     int chunk = 512;         // kets per CTA task
     std::vector<int4> tasks; // static FP64 task list
     int task_cap = 0;        // capacity of the per-build (mixed) lists
+    // small builds: the class runs as warp tasks (unit.cuh).  items[i].w is
+    // then the kets per task of item i, utasks the FP64 task list in order of
+    // decreasing lane time, ucap the capacity of the per-build lists
+    bool unit = false;
+    std::vector<int4> utasks;
+    int ucap = 0;
     // device copies
     int *d_bra = nullptr, *d_ket = nullptr, *d_bra_orig = nullptr, *d_ket_orig = nullptr;
     double *d_bra_x = nullptr, *d_ket_x = nullptr;
     double4 *d_ket_rec = nullptr;
     int4 *d_items = nullptr;
     int4 *d_tasks = nullptr;
+    int4 *d_utasks = nullptr;
     // mixed precision: per-build task lists
     int4 *d_tasks64 = nullptr, *d_tasks32 = nullptr;
     int *d_ntasks = nullptr;  // [0] fp64 count, [1] fp32 count, [2] fp32 quartets (lo), [3] (hi)
@@ -200,8 +207,9 @@ struct DeviceBuffers {
     double *D = nullptr, *F = nullptr;
     double *Dsq = nullptr;  // the build's D as a full n x n matrix (class kernels read it)
     float *Df = nullptr;    // FP32 tier: the same in single precision
-    // open-shell builds (made at the first one): the Coulomb and exchange
-    // densities as two consecutive full n x n matrices, and their float copies
+    // open-shell builds (made at the first one): the Coulomb density and the
+    // exchange densities of both spins as three consecutive full n x n
+    // matrices, and their float copies
     double *uhf_sq = nullptr;
     float *uhf_sqf = nullptr;
     long long *scratch_total = nullptr;  // device counters (mixed split)
@@ -233,8 +241,10 @@ struct LaunchCtx {
     // and the primitive screening cut (fp32_prim * fp32_cut; 0 = off)
     const unsigned long long *maxd = nullptr;
     double prim_cut = 0.0;
-    // open-shell builds: the exchange terms read a second full matrix at D + k_offset (0 = D itself)
+    // open-shell builds: the exchange terms read a further full matrix at D + k_offset (0 = D itself);
+    // warp-task launches of such a build evaluate both spins (k_offset, 2 k_offset; F and F2)
     size_t k_offset = 0;
+    double *F2 = nullptr;
     const double *rys_tab7 = nullptr;  // f classes: the 1..7-root table
 };
 
@@ -261,16 +271,42 @@ cudaError_t launch_batch_prep(const MolView *d_mols, int nmol, long long max_nsq
 cudaError_t launch_split_batch(int nitems, const int4 *items, const ClassView *d_cviews,
                                const unsigned long long *maxd, double fp32_cut, int chunk, int4 *tasks64,
                                int4 *tasks32, int *counts, cudaStream_t stream);
-// full n x n copy of a packed density, and its float copy when sqf is non-null
-cudaError_t launch_unpack(const double *packed, int n, double *sq, float *sqf, cudaStream_t st);
-// open-shell builds: sq = ca * A + cb * B from two packed matrices (full n x n, float copy when sqf)
-cudaError_t launch_unpack_combo(const double *pa, const double *pb, double ca, double cb, int n, double *sq,
-                                float *sqf, cudaStream_t st);
-cudaError_t launch_maxabs(const double *x, long long n, unsigned long long *out,
-                          cudaStream_t stream);
-cudaError_t launch_split_tasks(int nitems, const int4 *items, const double *bra_x, const double *ket_x,
-                               const unsigned long long *maxd, double fp32_cut, int chunk,
-                               int4 *tasks64, int4 *tasks32, int *counts, cudaStream_t stream);
+// start of a build in one launch: F zeroed, the density as a full n x n matrix
+// (and in float where sqf is non-null), the per-build task counters zeroed and,
+// where maxd is non-null (zeroed by the caller), max |D|.  Open-shell builds
+// (pb non-null): sq = pa + pb, then n*n and 2 n*n further the exchange
+// densities 2 pa and 2 pb, and F2 zeroed too.
+struct PrepArgs {
+    const double *pa, *pb;
+    double *sq;
+    float *sqf;
+    double *F, *F2;
+    unsigned long long *maxd;
+    int n;
+    int *counts[NKERN];  // four counters per class, or null
+};
+cudaError_t launch_prep(const PrepArgs &a, cudaStream_t st);
+// mixed precision: the FP64 and FP32 task lists of several classes in one launch
+struct SplitClass {
+    const int4 *items;
+    const double *bra_x, *ket_x;
+    int4 *tasks64, *tasks32;
+    int *counts;
+    int nitems, chunk, first_block;  // chunk 0: the item's own (items[i].w)
+};
+struct SplitArgs {
+    const unsigned long long *maxd;
+    double fp32_cut;
+    int ncls;
+    SplitClass cls[NKERN];
+};
+cudaError_t launch_split_tasks(SplitArgs a, cudaStream_t st);
+// the warp-task classes of a small build: one launch per register budget
+struct UnitArgs;
+constexpr int UNIT_PG[NKERN] = {1, 1, 1, 1, 1, 4, 1, 1, 1, 2, 2, 8, 4, 2, 8, 8, 8, 8, 8, 16, 16};  // pass lanes
+__host__ __device__ constexpr bool unit_low(int k) { return k <= 4 || (k >= 6 && k <= 8) || k == 10 || k == 13; }
+cudaError_t launch_units(bool low, int ncls, const int *ks, const LaunchCtx &ctx, const DevPlan *plans,
+                         const RankSplit *rs, int precision, int nbf);
 // Schwarz values of the f pair classes (sf, pf, df, ff) with the f classes'
 // shared-memory evaluation and the 1..7-root table (k_f.cu)
 cudaError_t launch_fschwarz(int pair_class, int npairs, int pair_off, const DevBasis &b, const double *rys_tab7,

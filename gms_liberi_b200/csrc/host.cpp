@@ -238,6 +238,7 @@ struct liberi_handle_s {
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     // small builds spread their classes over FAN_STREAMS streams (option "fan")
     bool fan_out = true;
+    bool units = true;  // warp tasks for the classes planned so (off while the tuner times the class kernels)
     cudaStream_t fan[FAN_STREAMS] = {};
     cudaEvent_t fan_ev[FAN_STREAMS] = {};
     int num_sms = 148;
@@ -570,6 +571,56 @@ static void balance_items(const PairsHost &pr, int rank, int nsize, PlanHost &ph
     build_tasks(ph);
 }
 
+// Small builds: which classes run as warp tasks (unit.cuh), and how many kets
+// a warp takes of each item.  UNIT_US is the time in microseconds that one
+// thread spends on a primitive quartet of the class, all passes, in the
+// thread-per-quartet kernels (class times of an ethane-shaped build over its
+// costliest quartet's primitive count).  With C the sum of that over the
+// build, an even spread over the GPU's resident lanes takes C / UNIT_LANES; a
+// class goes to warp tasks where its quartets cannot fill the lanes, or where
+// its costliest quartet alone would outlast that even spread.  An item's lanes
+// per quartet are the fewest that bring a quartet below half the even spread,
+// but not below UNIT_FLOOR_US, where a warp's own start and digestion dominate.
+static const double UNIT_US[NKERN] = {0.31, 0.40, 0.62, 0.80, 0.60, 4.0, 0.60, 0.80, 0.80, 1.3, 1.4,
+                                      6.2,  1.4,  1.5,  17.0, 20.0, 6.3, 7.8,  15.0, 60.0, 150.0};
+static const double UNIT_LANES = 148 * 16 * 32, UNIT_FLOOR_US = 5.0, UNIT_TAIL_US = 25.0;
+
+static void plan_units(const PairsHost &pr, PlanHost *plans) {
+    long long nquart = 0;
+    double total_us = 0.0, max_us[NKERN] = {};
+    for (int k = 0; k < NKERN; k++)
+        for (const int4 &it : plans[k].items) {
+            nquart += it.z;
+            const double us = UNIT_US[k] * pr.nprim[plans[k].bra_ids[it.x]] * pr.kab[plans[k].ket_ids[it.y]];
+            total_us += us * it.z;
+            max_us[k] = std::max(max_us[k], us);
+        }
+    if (nquart > FAN_MAX_QUARTETS) return;
+    const double even_us = total_us / UNIT_LANES, aim_us = std::max(0.5 * even_us, UNIT_FLOOR_US);
+    for (int k = 0; k < NKERN; k++) {
+        PlanHost &ph = plans[k];
+        if (ph.items.empty()) continue;
+        long long q = 0;
+        for (const int4 &it : ph.items) q += it.z;
+        if ((double)q * UNIT_PG[k] > UNIT_LANES && max_us[k] <= std::max(even_us, UNIT_TAIL_US)) continue;
+        ph.unit = true;
+        std::vector<std::pair<double, int4>> lst;
+        for (int4 &it : ph.items) {
+            const double us = UNIT_US[k] * pr.nprim[ph.bra_ids[it.x]] * pr.kab[ph.ket_ids[it.y]];
+            int g = UNIT_PG[k];
+            while (g < 32 && us > g * aim_us) g *= 2;
+            it.w = 32 / g;
+            for (int k0 = 0; k0 < it.z; k0 += it.w)
+                lst.push_back({us / g, make_int4(it.x, it.y + k0, std::min(it.w, it.z - k0), 0)});
+            ph.ucap += (it.z + it.w - 1) / it.w + 1;
+        }
+        std::stable_sort(lst.begin(), lst.end(), [](const std::pair<double, int4> &a, const std::pair<double, int4> &b) {
+            return a.first > b.first;
+        });
+        for (const auto &t : lst) ph.utasks.push_back(t.second);
+    }
+}
+
 // Every class's plan (and, for the balanced rank split, this rank's slice of
 // it) on up to one host thread per class: each reads the pairs and writes
 // only its own plan.  C60's 21 plans took 42 ms on one thread.
@@ -601,6 +652,7 @@ static void build_plans(const PairsHost &pr, double cut, const int *chunk, int r
     }
     worker();
     for (std::thread &th : pool) th.join();
+    plan_units(pr, plans);
 }
 
 static void make_tasks(const PlanHost &ph, int chunk, int mol, std::vector<int4> &out) {
@@ -653,8 +705,9 @@ static int upload_plans(liberi_handle h) {
         CUDA_TRY(dev_upload(h, &ph.d_ket_x, ph.ket_x.data(), ph.ket_x.size()));
         CUDA_TRY(dev_upload(h, &ph.d_items, ph.items.data(), ph.items.size()));
         CUDA_TRY(dev_upload(h, &ph.d_tasks, ph.tasks.data(), ph.tasks.size()));
-        CUDA_TRY(dev_alloc(h, &ph.d_tasks64, (size_t)ph.task_cap));
-        CUDA_TRY(dev_alloc(h, &ph.d_tasks32, (size_t)ph.task_cap));
+        CUDA_TRY(dev_upload(h, &ph.d_utasks, ph.utasks.data(), ph.utasks.size()));
+        CUDA_TRY(dev_alloc(h, &ph.d_tasks64, (size_t)std::max(ph.task_cap, ph.ucap)));
+        CUDA_TRY(dev_alloc(h, &ph.d_tasks32, (size_t)std::max(ph.task_cap, ph.ucap)));
         CUDA_TRY(dev_alloc(h, &ph.d_ntasks, 4));
     }
     return LIBERI_OK;
@@ -667,7 +720,8 @@ static size_t plan_device_bytes(const PlanHost &ph) {
            up_bytes(ph.ket_ids.size(), sizeof(int)) + up_bytes(ph.bra_orig.size(), sizeof(int)) +
            up_bytes(ph.ket_orig.size(), sizeof(int)) + up_bytes(ph.bra_x.size(), sizeof(double)) +
            up_bytes(ph.ket_x.size(), sizeof(double)) + up_bytes(ph.items.size(), sizeof(int4)) +
-           up_bytes(ph.tasks.size(), sizeof(int4)) + 2 * al_bytes((size_t)ph.task_cap, sizeof(int4)) +
+           up_bytes(ph.tasks.size(), sizeof(int4)) + up_bytes(ph.utasks.size(), sizeof(int4)) +
+           2 * al_bytes((size_t)std::max(ph.task_cap, ph.ucap), sizeof(int4)) +
            al_bytes(4, sizeof(int));
 }
 
@@ -854,7 +908,7 @@ static int replan(liberi_handle h) {
         // tuner uploaded on its own is released here
         for (void *p : {(void *)ph.d_ket_rec, (void *)ph.d_bra, (void *)ph.d_ket, (void *)ph.d_bra_orig,
                         (void *)ph.d_ket_orig, (void *)ph.d_bra_x, (void *)ph.d_ket_x, (void *)ph.d_items,
-                        (void *)ph.d_tasks, (void *)ph.d_tasks64, (void *)ph.d_tasks32, (void *)ph.d_ntasks})
+                        (void *)ph.d_tasks, (void *)ph.d_utasks, (void *)ph.d_tasks64, (void *)ph.d_tasks32, (void *)ph.d_ntasks})
             if (p) dev_release(h, p);
     }
     if (h->arena_plans.base) dev_release(h, h->arena_plans.base);
@@ -904,19 +958,19 @@ static DevPlan dev_plan_of(liberi_handle h, int k) {
 }
 
 // One Fock build on device buffers.  Closed shell (dDb null): F = J(D) - K(D)
-// in the reference's DIRFCK units.  Open shell (dDb non-null, spin 0 or 1):
+// in the reference's DIRFCK units.  Open shell (dDb, dFb non-null):
 // F_spin = J(D + Db) - K(2 D_spin), D the alpha density: the kernels read the
-// Coulomb density and, k_offset further on, the exchange density.
+// Coulomb density and, k_offset further on, the exchange density; warp-task
+// classes evaluate both spins from one set of integrals, the others run once
+// per spin.
 static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaStream_t st,
-                           const double *dDb = nullptr, int spin = 0) {
+                           const double *dDb = nullptr, double *dFb = nullptr) {
     if (h->plan_dirty) {
         int rc = replan(h);
         if (rc) return rc;
     }
     h->last_split_lists = h->precision == 1;
     const BasisHost &b = h->basis;
-    const long long ntri = (long long)b.num_bas * (b.num_bas + 1) / 2;
-    CUDA_TRY(cudaMemsetAsync(dF, 0, ntri * sizeof(double), st));  // liberi_driver.F90:64
     LaunchCtx ctx;
     ctx.basis = dev_basis(h);
     ctx.rys_tab = h->d_tab;
@@ -931,27 +985,56 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
     ctx.Df = h->dev.Df;
     ctx.maxd = mixed ? h->d_maxd : nullptr;
     ctx.prim_cut = mixed ? h->fp32_prim * h->fp32_cut : 0.0;
-    if (!dDb) {
-        // the class kernels read D as a full matrix (and in float for the FP32 tier)
-        CUDA_TRY(launch_unpack(dD, b.num_bas, h->dev.Dsq, mixed ? h->dev.Df : nullptr, st));
-        if (mixed) CUDA_TRY(launch_maxabs(dD, ntri, h->d_maxd, st));
-    } else {
+    if (dDb) {
         const size_t nsq = (size_t)b.num_bas * b.num_bas;
         if (!h->dev.uhf_sq) {  // first open-shell build of this handle
-            CUDA_TRY(cudaMallocAsync((void **)&h->dev.uhf_sq, 2 * nsq * sizeof(double), h->stream));
+            CUDA_TRY(cudaMallocAsync((void **)&h->dev.uhf_sq, 3 * nsq * sizeof(double), h->stream));
             h->allocs.push_back(h->dev.uhf_sq);
-            CUDA_TRY(cudaMallocAsync((void **)&h->dev.uhf_sqf, 2 * nsq * sizeof(float), h->stream));
+            CUDA_TRY(cudaMallocAsync((void **)&h->dev.uhf_sqf, 3 * nsq * sizeof(float), h->stream));
             h->allocs.push_back(h->dev.uhf_sqf);
             CUDA_TRY(cudaStreamSynchronize(h->stream));
         }
-        CUDA_TRY(launch_unpack_combo(dD, dDb, 1.0, 1.0, b.num_bas, h->dev.uhf_sq, mixed ? h->dev.uhf_sqf : nullptr, st));
-        CUDA_TRY(launch_unpack_combo(dD, dDb, spin == 0 ? 2.0 : 0.0, spin == 0 ? 0.0 : 2.0, b.num_bas,
-                                     h->dev.uhf_sq + nsq, mixed ? h->dev.uhf_sqf + nsq : nullptr, st));
-        // the mixed tier's bound uses the largest element of both densities
-        if (mixed) CUDA_TRY(launch_maxabs(h->dev.uhf_sq, (long long)(2 * nsq), h->d_maxd, st));
         ctx.D = h->dev.uhf_sq;
         ctx.Df = h->dev.uhf_sqf;
         ctx.k_offset = nsq;
+    }
+    const int nspin = dDb ? 2 : 1;
+    const size_t k_off = ctx.k_offset;
+    // classes that run once per spin: F and the exchange density of spin s
+    auto set_spin = [&](int s) {
+        ctx.F = s == 0 ? dF : dFb;
+        ctx.k_offset = (size_t)(s + 1) * k_off;
+    };
+    auto runs = [&](int k) { return h->plan[k].total != 0 && ((h->class_mask >> k) & 1u); };
+    const bool units = h->units && !h->timing;
+    {  // F zeroed (liberi_driver.F90:64), D as the class kernels read it
+        PrepArgs pa{};
+        pa.pa = dD;
+        pa.pb = dDb;
+        pa.sq = const_cast<double *>(ctx.D);
+        pa.sqf = mixed ? const_cast<float *>(ctx.Df) : nullptr;
+        pa.F = dF;
+        pa.F2 = dFb;
+        pa.n = b.num_bas;
+        if (mixed) {
+            // (the mixed tier's bound uses the largest element of both densities of an open-shell build)
+            CUDA_TRY(cudaMemsetAsync(h->d_maxd, 0, sizeof(unsigned long long), st));
+            pa.maxd = h->d_maxd;
+            for (int k = 0; k < NKERN; k++) pa.counts[k] = runs(k) ? h->plan[k].d_ntasks : nullptr;
+        }
+        CUDA_TRY(launch_prep(pa, st));
+    }
+    if (mixed) {  // every class's FP64 and FP32 task lists
+        SplitArgs sa{};
+        sa.maxd = h->d_maxd;
+        sa.fp32_cut = h->fp32_cut;
+        for (int k = 0; k < NKERN; k++) {
+            const PlanHost &ph = h->plan[k];
+            if (!runs(k)) continue;
+            sa.cls[sa.ncls++] = SplitClass{ph.d_items, ph.d_bra_x, ph.d_ket_x, ph.d_tasks64, ph.d_tasks32, ph.d_ntasks,
+                                           (int)ph.items.size(), units && ph.unit ? 0 : ph.chunk, 0};
+        }
+        CUDA_TRY(launch_split_tasks(sa, st));
     }
     for (int k = 0; k < NKERN; k++) h->ev_recorded[k] = false;
     // mixed precision: every class's FP64 task list (the few quartets above
@@ -974,32 +1057,27 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
     const bool fan = h->fan_out && h->overlap && !h->timing && nquart <= FAN_MAX_QUARTETS;
     const bool fork = h->overlap && !h->timing && !fan;
     const uint32_t side64 = mixed ? 0u : h->side_mask;
+    // fan builds: launch i goes to stream i mod FAN_STREAMS, stream 0 being
+    // the build's own; a further stream is forked at its first launch, and
+    // only the forked ones are joined
+    int nfanned = 0;
+    bool forked[FAN_STREAMS] = {};
+    auto fan_stream = [&](cudaStream_t *out) -> int {
+        const int i = nfanned++ % FAN_STREAMS;
+        *out = st;
+        if (!fan || i == 0) return LIBERI_OK;
+        if (!h->fan[i]) {
+            CUDA_TRY(cudaStreamCreateWithFlags(&h->fan[i], cudaStreamNonBlocking));
+            CUDA_TRY(cudaEventCreateWithFlags(&h->fan_ev[i], cudaEventDisableTiming));
+        }
+        if (!forked[i]) CUDA_TRY(cudaStreamWaitEvent(h->fan[i], h->fork_ev, 0));
+        forked[i] = true;
+        *out = h->fan[i];
+        return LIBERI_OK;
+    };
     if (fan) {
-        if (mixed)
-            for (int k = 0; k < NKERN; k++) {
-                PlanHost &ph = h->plan[k];
-                if (ph.total == 0 || !((h->class_mask >> k) & 1u)) continue;
-                CUDA_TRY(launch_split_tasks((int)ph.items.size(), ph.d_items, ph.d_bra_x, ph.d_ket_x, h->d_maxd,
-                                            h->fp32_cut, ph.chunk, ph.d_tasks64, ph.d_tasks32, ph.d_ntasks, st));
-            }
         if (!h->fork_ev) CUDA_TRY(cudaEventCreateWithFlags(&h->fork_ev, cudaEventDisableTiming));
         CUDA_TRY(cudaEventRecord(h->fork_ev, st));
-        for (int i = 0; i < FAN_STREAMS; i++) {
-            if (!h->fan[i]) {
-                CUDA_TRY(cudaStreamCreateWithFlags(&h->fan[i], cudaStreamNonBlocking));
-                CUDA_TRY(cudaEventCreateWithFlags(&h->fan_ev[i], cudaEventDisableTiming));
-            }
-            CUDA_TRY(cudaStreamWaitEvent(h->fan[i], h->fork_ev, 0));
-        }
-    }
-    int nfanned = 0;
-    if (fork && mixed) {
-        for (int k = 0; k < NKERN; k++) {
-            PlanHost &ph = h->plan[k];
-            if (ph.total == 0 || !((h->class_mask >> k) & 1u)) continue;
-            CUDA_TRY(launch_split_tasks((int)ph.items.size(), ph.d_items, ph.d_bra_x, ph.d_ket_x, h->d_maxd,
-                                        h->fp32_cut, ph.chunk, ph.d_tasks64, ph.d_tasks32, ph.d_ntasks, st));
-        }
     }
     if (fork) {
         // each object is created once per handle (the fan-out path may have
@@ -1012,10 +1090,36 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
     }
     // high-L classes (few quartets per row pair, a latency tail) first
     static const int ORDER[NKERN] = {20, 19, 18, 14, 11, 13, 10, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 15, 16, 17};
+    // warp-task classes: one launch per register budget and precision, the
+    // high-L ones (longest tasks) first
+    for (int low = 0; low < 2 && units; low++)
+        for (int prec = 0; prec < (mixed ? 2 : 1); prec++) {
+            int ks[NKERN], n = 0;
+            DevPlan dps[NKERN];
+            RankSplit rss[NKERN];
+            for (int oi = 0; oi < NKERN; oi++) {
+                const int k = ORDER[oi];
+                const PlanHost &ph = h->plan[k];
+                if (!runs(k) || !ph.unit || unit_low(k) != (low == 1)) continue;
+                DevPlan dp = dev_plan_of(h, k);
+                dp.tasks = !mixed ? ph.d_utasks : (prec == 0 ? ph.d_tasks64 : ph.d_tasks32);
+                dp.ntasks_dev = mixed ? ph.d_ntasks + prec : nullptr;
+                dp.ntasks = mixed ? ph.ucap : (int)ph.utasks.size();
+                ks[n] = k;
+                rss[n] = rank_split_of(h, k);
+                dps[n++] = dp;
+            }
+            if (n == 0) continue;
+            int rc = fan_stream(&ctx.stream);
+            if (rc) return rc;
+            ctx.F2 = dFb;
+            CUDA_TRY(launch_units(low == 1, n, ks, ctx, dps, rss, prec, b.num_bas));
+        }
+    ctx.stream = st;
     for (int oi = 0; oi < NKERN; oi++) {
         const int k = ORDER[oi];
         PlanHost &ph = h->plan[k];
-        if (ph.total == 0 || !((h->class_mask >> k) & 1u)) continue;
+        if (!runs(k) || (units && ph.unit)) continue;
         const KernelDesc &kd = KDESC[k];
         ctx.stream = st;
         if (h->timing) {
@@ -1030,44 +1134,30 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
         const int nbf = b.num_bas;
         const size_t tile_bytes = (size_t)(ncart_l(kd.la) + ncart_l(kd.lb)) * nbf * sizeof(double);
         const int tile_rows = (tile_bytes <= TILE_MAX_BYTES && ((h->tile_mask >> k) & 1u)) ? 1 : 0;
-        if (fan) {  // every launch of the class on its fan stream (task splits came first)
-            ctx.stream = h->fan[nfanned++ % FAN_STREAMS];
-            if (!mixed) {
-                dp.tasks = ph.d_tasks;
-                dp.ntasks_dev = nullptr;
-                dp.ntasks = (int)ph.tasks.size();
-                CUDA_TRY(launch_class(k, ctx, dp, rs, 0, nbf, tile_rows, h->variant[0][k]));
-            } else {
-                dp.ntasks = ph.task_cap;
-                dp.tasks = ph.d_tasks64;
-                dp.ntasks_dev = ph.d_ntasks;
-                CUDA_TRY(launch_class(k, ctx, dp, rs, 0, nbf, tile_rows, h->variant[0][k]));
+        // fan builds: every launch of the class on its fan stream; others on
+        // the build's stream, FP64 lists of mixed builds and the classes of
+        // side_mask on the side stream
+        cudaStream_t s64 = (fork && (mixed || ((side64 >> k) & 1u))) ? h->side : st, s32 = st;
+        if (fan) {
+            int rc = fan_stream(&s64);
+            if (rc) return rc;
+            s32 = s64;
+        }
+        for (int s = 0; s < nspin; s++) {
+            set_spin(s);
+            dp.tasks = mixed ? ph.d_tasks64 : ph.d_tasks;
+            dp.ntasks_dev = mixed ? ph.d_ntasks : nullptr;
+            dp.ntasks = mixed ? ph.task_cap : (int)ph.tasks.size();
+            ctx.stream = s64;
+            CUDA_TRY(launch_class(k, ctx, dp, rs, 0, nbf, tile_rows, h->variant[0][k]));
+            if (mixed) {
                 dp.tasks = ph.d_tasks32;
                 dp.ntasks_dev = ph.d_ntasks + 1;
+                ctx.stream = s32;
                 CUDA_TRY(launch_class(k, ctx, dp, rs, 1, nbf, tile_rows, h->variant[1][k]));
             }
-            ctx.stream = st;
-        } else if (!mixed) {
-            dp.tasks = ph.d_tasks;
-            dp.ntasks_dev = nullptr;
-            dp.ntasks = (int)ph.tasks.size();
-            ctx.stream = (fork && ((side64 >> k) & 1u)) ? h->side : st;
-            CUDA_TRY(launch_class(k, ctx, dp, rs, 0, nbf, tile_rows, h->variant[0][k]));
-            ctx.stream = st;
-        } else {
-            if (!fork)  // (fan and fork builds split every class first)
-                CUDA_TRY(launch_split_tasks((int)ph.items.size(), ph.d_items, ph.d_bra_x, ph.d_ket_x, h->d_maxd,
-                                            h->fp32_cut, ph.chunk, ph.d_tasks64, ph.d_tasks32, ph.d_ntasks, st));
-            dp.ntasks = ph.task_cap;
-            dp.tasks = ph.d_tasks64;
-            dp.ntasks_dev = ph.d_ntasks;
-            ctx.stream = fork ? h->side : st;
-            CUDA_TRY(launch_class(k, ctx, dp, rs, 0, nbf, tile_rows, h->variant[0][k]));
-            dp.tasks = ph.d_tasks32;
-            dp.ntasks_dev = ph.d_ntasks + 1;
-            ctx.stream = st;
-            CUDA_TRY(launch_class(k, ctx, dp, rs, 1, nbf, tile_rows, h->variant[1][k]));
         }
+        ctx.stream = st;
         if (h->timing) {
             CUDA_TRY(cudaEventRecord(h->ev[k][1], st));
             h->ev_recorded[k] = true;
@@ -1080,13 +1170,18 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
             PlanHost &ph = h->plan[k];
             if (ph.total == 0) continue;
             DevPlan dp = dev_plan_of(h, k);
-            ctx.stream = fan ? h->fan[nfanned++ % FAN_STREAMS] : st;
-            CUDA_TRY(launch_fclass(k, ctx, dp, rank_split_of(h, k), b.num_bas));
+            int rc = fan_stream(&ctx.stream);
+            if (rc) return rc;
+            for (int s = 0; s < nspin; s++) {
+                set_spin(s);
+                CUDA_TRY(launch_fclass(k, ctx, dp, rank_split_of(h, k), b.num_bas));
+            }
         }
         ctx.stream = st;
     }
     if (fan)  // join: the build completes on the caller's stream
-        for (int i = 0; i < FAN_STREAMS; i++) {
+        for (int i = 1; i < FAN_STREAMS; i++) {
+            if (!forked[i]) continue;
             CUDA_TRY(cudaEventRecord(h->fan_ev[i], h->fan[i]));
             CUDA_TRY(cudaStreamWaitEvent(st, h->fan_ev[i], 0));
         }
@@ -1467,8 +1562,7 @@ int liberi_c_fock_build_uhf_device(liberi_handle h, const double *d_density_a, c
     DeviceGuard dev_guard(h->device);
     CUDA_TRY(dev_guard.err);
     cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
-    int rc = build_on_device(h, d_density_a, d_fock_a, st, d_density_b, 0);
-    if (!rc) rc = build_on_device(h, d_density_a, d_fock_b, st, d_density_b, 1);
+    int rc = build_on_device(h, d_density_a, d_fock_a, st, d_density_b, d_fock_b);
     if (rc) return rc;
     CUDA_TRY(cudaGetLastError());
     return LIBERI_OK;
@@ -1494,10 +1588,7 @@ int liberi_c_fock_build_uhf(liberi_handle h, const double *density_a, const doub
     cudaError_t e = cudaMemcpyAsync(h->dev.D, density_a, bytes, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(db, density_b, bytes, cudaMemcpyHostToDevice, st);
     int rc = LIBERI_OK;
-    if (e == cudaSuccess) {
-        rc = build_on_device(h, h->dev.D, h->dev.F, st, db, 0);
-        if (!rc) rc = build_on_device(h, h->dev.D, fb, st, db, 1);
-    }
+    if (e == cudaSuccess) rc = build_on_device(h, h->dev.D, h->dev.F, st, db, fb);
     if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(fock_a, h->dev.F, bytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(fock_b, fb, bytes, cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(db, st);
@@ -1785,6 +1876,7 @@ int liberi_c_autotune(liberi_handle h, int32_t reps, int32_t *chunks_out) {
     const uint32_t mask0 = h->class_mask;
     const int prec0 = h->precision;
     const double cut0 = h->fp32_cut;
+    h->units = false;
     int rc = LIBERI_OK;
     // time one configuration of class k: reps builds of that class alone
     auto time_class = [&](int k, float *ms) -> int {
@@ -1855,6 +1947,7 @@ int liberi_c_autotune(liberi_handle h, int32_t reps, int32_t *chunks_out) {
             h->fp32_cut = cut0;
         }
     }
+    h->units = true;
     h->class_mask = mask0;
     h->precision = prec0;
     h->fp32_cut = cut0;
@@ -2007,7 +2100,7 @@ static int quartet_fingerprint(liberi_handle h, int nclass, uint64_t *out) {
             continue;
         }
         // the lists the last (mixed-precision) build split and launched
-        dp.ntasks = ph.task_cap;
+        dp.ntasks = std::max(ph.task_cap, ph.ucap);
         dp.tasks = ph.d_tasks64;
         dp.ntasks_dev = ph.d_ntasks;
         e = launch_quartet_fp(k, ctx, dp, rs, d_out + 3 * k);

@@ -1,7 +1,7 @@
 // kernels.cu -- class dispatch, Schwarz generator and mixed-precision task
 // builder of the Fock-build engine; the class kernels themselves are
 // instantiated in k_*.cu from quartet.cuh.
-#include "quartet.cuh"
+#include "unit.cuh"
 
 namespace liberi {
 
@@ -43,15 +43,6 @@ __global__ void __launch_bounds__(64) prim_bound_kernel(DevBasis b, int pair_off
     }
 }
 
-__global__ void maxabs_kernel(const double *x, long long n, unsigned long long *out) {
-    double m = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        m = fmax(m, fabs(x[i]));
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
-}
-
 // Per plan item (bra, ket segment, surviving count): split = number of its
 // kets with x_bra*x_ket*max|D| >= fp32_cut (a prefix, the segment is sorted
 // by x); FP64 tasks cover [0, split), FP32 tasks [split, count).  One CTA
@@ -71,22 +62,12 @@ __device__ __forceinline__ int item_split(const int4 &it, const double *bra_x, c
 // One thread per item: the split point, then output ranges reserved with
 // atomics (task order only affects load balance).  counts[0..1]: FP64 and
 // FP32 task counts, counts[2..3]: FP32 quartet count (64-bit, low word first);
-// zeroed before the launch.  BATCH: item.w is the molecule, whose Schwarz
-// lists and max|D| are used and which the tasks carry; else one molecule.
-template <bool BATCH>
-__global__ void __launch_bounds__(256) split_tasks_kernel(int nitems, const int4 *items, const double *bra_x1,
-                                                          const double *ket_x1, const ClassView *cviews,
-                                                          const unsigned long long *maxd_bits, double fp32_cut,
-                                                          int chunk, int4 *tasks64, int4 *tasks32, int *counts) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    const int4 it = items[i];
-    const double *bx = BATCH ? cviews[it.w].bra_x : bra_x1;
-    const double *kx = BATCH ? cviews[it.w].ket_x : ket_x1;
-    const double maxd = __longlong_as_double((long long)maxd_bits[BATCH ? it.w : 0]);
+// zeroed before the launch.
+__device__ __forceinline__ void split_item(const int4 &it, const double *bx, const double *kx, double maxd,
+                                           double fp32_cut, int chunk, int4 *tasks64, int4 *tasks32, int *counts,
+                                           int w) {
     const int s = item_split(it, bx, kx, maxd, fp32_cut);
     const int n64 = (s + chunk - 1) / chunk, n32 = (it.z - s + chunk - 1) / chunk;
-    const int w = BATCH ? it.w : 0;
     if (n64) {
         int o = atomicAdd(counts, n64);
         for (int k = 0; k < s; k += chunk) tasks64[o++] = make_int4(it.x, it.y + k, min(chunk, s - k), w);
@@ -96,6 +77,29 @@ __global__ void __launch_bounds__(256) split_tasks_kernel(int nitems, const int4
         for (int k = s; k < it.z; k += chunk) tasks32[o++] = make_int4(it.x, it.y + k, min(chunk, it.z - k), w);
         atomicAdd(reinterpret_cast<unsigned long long *>(counts + 2), (unsigned long long)(it.z - s));
     }
+}
+// batch: item.w is the molecule, whose Schwarz lists and max|D| are used and
+// which the tasks carry
+__global__ void __launch_bounds__(256) split_batch_kernel(int nitems, const int4 *items, const ClassView *cviews,
+                                                          const unsigned long long *maxd_bits, double fp32_cut,
+                                                          int chunk, int4 *tasks64, int4 *tasks32, int *counts) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nitems) return;
+    const int4 it = items[i];
+    split_item(it, cviews[it.w].bra_x, cviews[it.w].ket_x, __longlong_as_double((long long)maxd_bits[it.w]), fp32_cut,
+               chunk, tasks64, tasks32, counts, it.w);
+}
+// one molecule: every class of the build in one launch (21 launches and 21
+// counter resets cost a 10-atom mixed build about 100 us of host time)
+__global__ void __launch_bounds__(256) split_tasks_kernel(const __grid_constant__ SplitArgs a) {
+    int c = 0;
+    while (c + 1 < a.ncls && (int)blockIdx.x >= a.cls[c + 1].first_block) c++;
+    const SplitClass &s = a.cls[c];
+    const int i = ((int)blockIdx.x - s.first_block) * blockDim.x + threadIdx.x;
+    if (i >= s.nitems) return;
+    const int4 it = s.items[i];
+    split_item(it, s.bra_x, s.ket_x, __longlong_as_double((long long)a.maxd[0]), a.fp32_cut, s.chunk ? s.chunk : it.w,
+               s.tasks64, s.tasks32, s.counts, 0);
 }
 
 cudaError_t launch_prim_bound(int pc, int npairs, int pair_off, const DevBasis &b, const double *tab, float *out,
@@ -256,48 +260,46 @@ cudaError_t launch_class_batch(int k, const LaunchCtx &ctx, const int4 *tasks, i
     return cudaErrorInvalidValue;
 }
 
-__global__ void unpack_kernel(const double *__restrict__ packed, unsigned n, double *__restrict__ sq,
-                              float *__restrict__ sqf) {
-    const long long total = (long long)n * n;  // n <= 65535: an index fits unsigned 32-bit
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += stride) {
-        const unsigned i = (unsigned)g, r = i / n, c = i - r * n;
-        const double d = packed[tri0(r, c)];
-        sq[i] = d;
-        if (sqf) sqf[i] = (float)d;
+__global__ void __launch_bounds__(256) prep_kernel(const __grid_constant__ PrepArgs a) {
+    const unsigned n = (unsigned)a.n;  // n <= 65535: an index fits unsigned 32-bit
+    const long long total = (long long)n * n, ntri = (long long)n * (n + 1) / 2;
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    if (t0 < NKERN && a.counts[t0])
+        for (int i = 0; i < 4; i++) a.counts[t0][i] = 0;
+    for (long long g = t0; g < ntri; g += stride) {
+        a.F[g] = 0.0;
+        if (a.F2) a.F2[g] = 0.0;
     }
-}
-
-// Open-shell builds: sq = ca * A + cb * B as a full n x n matrix (and its float copy)
-__global__ void unpack_combo_kernel(const double *__restrict__ pa, const double *__restrict__ pb, double ca,
-                                    double cb, unsigned n, double *__restrict__ sq, float *__restrict__ sqf) {
-    const long long total = (long long)n * n;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += stride) {
-        const unsigned i = (unsigned)g, r = i / n, c = i - r * n;
-        const unsigned t = tri0(r, c);
-        const double d = ca * pa[t] + cb * pb[t];
-        sq[i] = d;
-        if (sqf) sqf[i] = (float)d;
+    double mx = 0.0;
+    for (long long g = t0; g < total; g += stride) {
+        const unsigned i = (unsigned)g, r = i / n, c = i - r * n, t = tri0(r, c);
+        double d = a.pa[t];
+        if (a.pb) {
+            const double e = a.pb[t], xa = 2.0 * d, xb = 2.0 * e;
+            d += e;
+            a.sq[total + g] = xa;
+            a.sq[2 * total + g] = xb;
+            if (a.sqf) {
+                a.sqf[total + g] = (float)xa;
+                a.sqf[2 * total + g] = (float)xb;
+            }
+            mx = fmax(mx, fmax(fabs(xa), fabs(xb)));
+        }
+        a.sq[i] = d;
+        if (a.sqf) a.sqf[i] = (float)d;
+        mx = fmax(mx, fabs(d));
     }
+    if (!a.maxd) return;
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(a.maxd, (unsigned long long)__double_as_longlong(mx));
 }
 
-cudaError_t launch_unpack_combo(const double *pa, const double *pb, double ca, double cb, int n, double *sq,
-                                float *sqf, cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
+cudaError_t launch_prep(const PrepArgs &a, cudaStream_t st) {
+    if (a.n <= 0) return cudaSuccess;
     const int threads = 256;
-    const long long want = ((long long)n * n + threads - 1) / threads;
+    const long long want = ((long long)a.n * a.n + threads - 1) / threads;
     const int blocks = (int)(want < 148LL * 8 ? want : 148LL * 8);
-    unpack_combo_kernel<<<blocks, threads, 0, st>>>(pa, pb, ca, cb, (unsigned)n, sq, sqf);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_unpack(const double *packed, int n, double *sq, float *sqf, cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    const int threads = 256;
-    const long long want = ((long long)n * n + threads - 1) / threads;
-    const int blocks = (int)(want < 148LL * 8 ? want : 148LL * 8);
-    unpack_kernel<<<blocks, threads, 0, st>>>(packed, (unsigned)n, sq, sqf);
+    prep_kernel<<<blocks, threads, 0, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -369,24 +371,64 @@ cudaError_t launch_schwarz(int pc, int npairs, int pair_off, const DevBasis &b, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_maxabs(const double *x, long long n, unsigned long long *out, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(out, 0, sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return e;
-    long long blocks = (n + 255) / 256;
-    if (blocks > 1184) blocks = 1184;
-    if (blocks < 1) blocks = 1;
-    maxabs_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, n, out);
+cudaError_t launch_split_tasks(SplitArgs a, cudaStream_t st) {
+    int blocks = 0;
+    for (int c = 0; c < a.ncls; c++) {
+        a.cls[c].first_block = blocks;
+        blocks += (a.cls[c].nitems + 255) / 256;
+    }
+    if (blocks == 0) return cudaSuccess;
+    split_tasks_kernel<<<(unsigned)blocks, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_split_tasks(int nitems, const int4 *items, const double *bra_x, const double *ket_x,
-                               const unsigned long long *maxd, double fp32_cut, int chunk, int4 *tasks64,
-                               int4 *tasks32, int *counts, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(counts, 0, 4 * sizeof(int), st);
-    if (e != cudaSuccess || nitems <= 0) return e;
-    split_tasks_kernel<false><<<(nitems + 255) / 256, 256, 0, st>>>(nitems, items, bra_x, ket_x, nullptr, maxd,
-                                                                    fp32_cut, chunk, tasks64, tasks32, counts);
-    return cudaGetLastError();
+extern template cudaError_t launch_unit_t<true, double>(const UnitArgs &, int, cudaStream_t);
+extern template cudaError_t launch_unit_t<true, float>(const UnitArgs &, int, cudaStream_t);
+extern template cudaError_t launch_unit_t<false, double>(const UnitArgs &, int, cudaStream_t);
+extern template cudaError_t launch_unit_t<false, float>(const UnitArgs &, int, cudaStream_t);
+
+cudaError_t launch_units(bool low, int ncls, const int *ks, const LaunchCtx &ctx, const DevPlan *plans,
+                         const RankSplit *rs, int precision, int nbf) {
+    UnitArgs a{};
+    a.b = ctx.basis;
+    a.tab = ctx.rys_tab;
+    a.tabf = ctx.rys_tabf;
+    a.Dm = ctx.D;
+    a.Dmf = ctx.Df;
+    a.F = ctx.F;
+    a.F2 = ctx.F2;
+    a.k_offset = ctx.k_offset;
+    a.maxd = ctx.maxd;
+    a.prim_cut = ctx.prim_cut;
+    a.nbf = nbf;
+    int blocks = 0;
+    for (int i = 0; i < ncls; i++) {
+        const DevPlan &dp = plans[i];
+        if (dp.ntasks <= 0) continue;
+        const KernelDesc &kd = KDESC[ks[i]];
+        UnitClass &u = a.cls[a.ncls++];
+        u.bra_ids = dp.bra_ids;
+        u.ket_rec = dp.ket_rec;
+        u.bra_orig = dp.bra_orig;
+        u.ket_orig = dp.ket_orig;
+        u.tasks = dp.tasks;
+        u.ntasks_dev = dp.ntasks_dev;
+        u.ntasks = dp.ntasks;
+        u.first_block = blocks;
+        u.cut = kd.digest_schwarz ? ctx.schwarz_cut : ctx.eri_cut;
+        u.thr = kd.asym;
+        u.k = ks[i];
+        u.strict = !kd.rys;
+        u.swapped = dp.swapped ? 1 : 0;
+        u.rs = rs[i];
+        blocks += (dp.ntasks + UNIT_WARPS - 1) / UNIT_WARPS;
+    }
+    if (blocks == 0) return cudaSuccess;
+    if (low)
+        return precision == 0 ? launch_unit_t<true, double>(a, blocks, ctx.stream)
+                              : launch_unit_t<true, float>(a, blocks, ctx.stream);
+    return precision == 0 ? launch_unit_t<false, double>(a, blocks, ctx.stream)
+                          : launch_unit_t<false, float>(a, blocks, ctx.stream);
 }
 
 cudaError_t launch_split_batch(int nitems, const int4 *items, const ClassView *d_cviews,
@@ -394,8 +436,8 @@ cudaError_t launch_split_batch(int nitems, const int4 *items, const ClassView *d
                                int4 *tasks32, int *counts, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(counts, 0, 4 * sizeof(int), st);
     if (e != cudaSuccess || nitems <= 0) return e;
-    split_tasks_kernel<true><<<(nitems + 255) / 256, 256, 0, st>>>(nitems, items, nullptr, nullptr, d_cviews, maxd,
-                                                                   fp32_cut, chunk, tasks64, tasks32, counts);
+    split_batch_kernel<<<(nitems + 255) / 256, 256, 0, st>>>(nitems, items, d_cviews, maxd, fp32_cut, chunk, tasks64,
+                                                             tasks32, counts);
     return cudaGetLastError();
 }
 

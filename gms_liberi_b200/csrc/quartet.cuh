@@ -28,6 +28,7 @@
 // times max|D| falls below the mixed-precision cut; step 2 always digests in
 // FP64.
 #pragma once
+#include <atomic>
 #include <cstdio>
 #include <type_traits>
 
@@ -1673,6 +1674,26 @@ __device__ __forceinline__ double schwarz_diag(const DevBasis &b, int P, const d
     return sqrt(m);
 }
 
+// A kernel's shared-memory limit and carveout (percent; -1: left alone), set
+// again only when they change: two runtime calls a launch cost as much host
+// time as the launch.  Per device; the values are hints of the launch that
+// asked last, as they were when every launch set them.
+struct FuncAttrs {
+    static constexpr int NDEV = 64;
+    std::atomic<int> last[NDEV];  // carveout + 2, 0 = never set (static storage)
+    cudaError_t set(const void *f, int smem_max, int carve) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        if (dev < NDEV && last[dev].load(std::memory_order_acquire) == carve + 2) return cudaSuccess;
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+        if (e != cudaSuccess) return e;
+        if (carve >= 0) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+        if (e == cudaSuccess && dev < NDEV) last[dev].store(carve + 2, std::memory_order_release);
+        return e;
+    }
+};
+
 template <int LA, int LB, int LC, int LD, typename R, bool BATCH, int V>
 cudaError_t launch_shape(const ClassArgs &a, cudaStream_t st) {
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
@@ -1691,16 +1712,14 @@ cudaError_t launch_shape(const ClassArgs &a, cudaStream_t st) {
     const size_t smem = (args.tile_rows ? tile_bytes : 0) + slot_bytes + STB;
     // the opt-in limit is raised to the per-CTA maximum, not to this launch's
     // size: a captured graph may hold a larger launch
-    cudaError_t e = cudaFuncSetAttribute(class_kernel<LA, LB, LC, LD, R, BATCH, V>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, CLASS_DYN_SMEM_MAX);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     // the rest of the SM's 256 KB stays L1 (the class's Rys table rows, pair
     // data and D): a shared-memory carveout of what MINB resident CTAs use
     {
         const size_t need = smem * (size_t)MINB;
         const int carve = need == 0 ? 0 : (int)std::min<size_t>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024));
-        e = cudaFuncSetAttribute(class_kernel<LA, LB, LC, LD, R, BATCH, V>,
-                                 cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+        static FuncAttrs attrs;
+        e = attrs.set((const void *)class_kernel<LA, LB, LC, LD, R, BATCH, V>, CLASS_DYN_SMEM_MAX, carve);
         if (e != cudaSuccess) return e;
     }
     class_kernel<LA, LB, LC, LD, R, BATCH, V><<<(unsigned)a.ntasks, CLASS_THREADS, smem, st>>>(args);

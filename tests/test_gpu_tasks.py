@@ -1,0 +1,104 @@
+"""Work splits of the small-build and f kernels at their edges, against the oracle.
+
+Warp tasks split a quartet over lanes by passes, primitive quartets and roots;
+f groups take a fixed number of (primitive quartet, root) units a round.  The
+molecules here have odd and uneven contractions on every angular momentum, so
+that the splits have remainders, next to uncontracted shells, where a quartet
+has fewer primitives than lanes.  Tolerance 1e-10 on F as for every FP64
+comparison with the oracle (integrals within 1e-11 of the cut may be kept on one
+side only).
+"""
+import numpy as np
+import pytest
+
+from gms_liberi_b200 import liberi
+from gms_liberi_b200 import molecules as M
+from oracle import oracle
+from test_gpu_parity import TOL_F, energy, gpu_fock
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {
+    # one shell: single quartets, every lane on one of them
+    "one_s": ([("s", 5)], None),
+    "one_d": ([("d", 3)], None),
+    # uneven contractions next to uncontracted shells
+    "mixed": ([("s", 7), ("sp", 2), ("p", 5), ("d", 3), ("d", 1)], [("s", 3), ("s", 1), ("p", 1)]),
+    # f shells with contracted partners: several rounds, a last one partly filled
+    "f": ([("s", 5), ("p", 3), ("d", 2), ("f", 3), ("f", 1)], [("s", 2), ("p", 1)]),
+}
+
+
+def _molecule(name, natoms):
+    heavy, light = SHAPES[name]
+    xyz = np.array([[0.0, 0.0, 0.0], [1.9, 0.4, -0.3], [-0.8, 2.3, 1.1], [0.5, -1.2, 9.0]])[:natoms]
+    sym = ["O", "C" if light is None else "H", "C", "H" if light else "C"][:natoms]
+
+    def shells(s):
+        return M.element_basis(s, light if s == "H" and light else heavy, 0.2, 60.0, seed=5)
+
+    b = M.build_basis(sym, xyz, shells)
+    b["schwrz"] = oracle.schwarz(b)
+    return b
+
+
+@pytest.mark.parametrize("name,natoms", [("one_s", 1), ("one_d", 1), ("one_d", 2), ("mixed", 1), ("mixed", 4),
+                                         ("f", 1), ("f", 3)])
+def test_small_builds_match_oracle(name, natoms):
+    b = _molecule(name, natoms)
+    D = M.density(b["num_bas"], max(1, b["num_bas"] // 3), seed=2)
+    Fo = oracle.fock_build(b, D)
+    F, st = gpu_fock(b, D)
+    assert np.abs(F - Fo).max() <= TOL_F
+    # the thread-per-quartet kernels (per-class timing keeps every class on them)
+    Fc, stc = gpu_fock(b, D, timing=1)
+    assert np.abs(Fc - Fo).max() <= TOL_F
+    assert (st["fingerprint"] == stc["fingerprint"]).all()
+    # mixed precision: the same set over both tiers, both kernel families
+    for timing in (0, 1):
+        Fm, stm = gpu_fock(b, D, precision=1, fp32_cut=1e-4, timing=timing)
+        assert abs(energy(D, Fm) - energy(D, Fo)) <= 1e-6
+        assert (stm["fingerprint"] == st["fingerprint"]).all()
+
+
+@pytest.mark.parametrize("name", ["mixed", "f"])
+def test_small_open_shell_builds_match_oracle(name):
+    b = _molecule(name, 3)
+    Da = M.density(b["num_bas"], 4, seed=3) * 0.5
+    Db = M.density(b["num_bas"], 3, seed=4) * 0.5
+    ref = oracle.fock_build_uhf(b, Da, Db)
+    for opts in ({}, {"timing": 1}, {"fan": 0}, {"precision": 1, "fp32_cut": 1e-6}):
+        h = liberi.liberi_create()
+        for k, v in opts.items():
+            h.set_option(k, v)
+        liberi.setup_from_basis(h, b)
+        for F, Fo in zip(liberi.fock_uhf(h, Da, Db), ref):
+            assert np.abs(F - Fo).max() <= (TOL_F if "precision" not in opts else 1e-8)
+        liberi.liberi_destroy(h)
+
+
+@pytest.mark.parametrize("name,natoms", [("one_s", 1), ("mixed", 4), ("f", 4)])
+def test_schwarz_of_uneven_contractions(name, natoms):
+    b = _molecule(name, natoms)
+    np.testing.assert_allclose(liberi.schwarz(b), b["schwrz"], rtol=1e-10, atol=1e-14)
+
+
+def test_schwarz_of_shells_sharing_exponents():
+    # an s and a p shell that name the same exponents (one sh_loc)
+    b = M.h2o_like()
+    s, p = [k for k in range(b["nsh"]) if b["atom_num"][k] == 1][-2:]
+    lo_s, lo_p, n = b["sh_loc"][s] - 1, b["sh_loc"][p] - 1, b["contr_num"][p]
+    assert b["ang_mom"][s] == 1 and b["ang_mom"][p] == 2
+    ref = liberi.schwarz(b)
+    b["coef_p"][lo_s:lo_s + n] = b["coef_p"][lo_p:lo_p + n]
+    b["sh_loc"][p] = b["sh_loc"][s]
+    np.testing.assert_array_equal(liberi.schwarz(b), ref)
+
+
+def test_rank_split_of_warp_tasks():
+    b = _molecule("mixed", 4)
+    D = M.density(b["num_bas"], 8, seed=6)
+    full = oracle.fock_build(b, D)
+    for split in (0, 1):
+        part = sum(gpu_fock(b, D, rank=r, nproc=3, rank_split=split)[0] for r in range(3))
+        assert np.abs(part - full).max() <= TOL_F
