@@ -3,70 +3,62 @@
 // the generated Rys kernels, src/rhf/eric, src/rhf/rys).
 //
 // An f quartet is too large for the thread-per-quartet class kernels ((ff|ff)
-// holds 10,000 integrals and 7 roots), so a group of threads evaluates one
-// shell quartet at a time, everything in shared memory, with the class's
-// angular momenta as compile-time parameters (one instantiation per class).
-// The group is one warp (four tasks per CTA, warp barriers only) where the
-// quartet's working set fits 24 KB, else a whole 256-thread CTA:
-//   1. 3 n threads per primitive quartet (one per root and Cartesian axis)
-//      take the root and weight from the 7-root table and run the 2D vertical
-//      recurrence g[e][f], e <= la+lb, f <= lc+ld (prefactor and weight folded
-//      into the x axis);
-//   2. all threads expand g to the 2D integrals I[a][b][c][d] by the closed
-//      form of the transfer relation, I = sum_i sum_k C(b,i) AB^(b-i) C(d,k)
-//      CD^(d-k) g[a+i][c+k];
-//   3. every thread accumulates its own Cartesian components of the shell
-//      quartet, sum_r Ix Iy Iz, into the block in shared memory.
-// Several primitive quartets share one round when shared memory allows.
-// After the last primitive quartet every thread digests its own components
-// with the DIRFCK rules (unique components for equal shells, 0.5 factors on
-// equal functions, the six packed updates, src/rhf/rys/int3011_rysgen.F90
-// digestion) by FP64 atomics, reading D from the build's full matrix.
-// FP64 only: a mixed-precision build runs its f classes in FP64.
+// holds 10,000 integrals and 7 roots), so a group of warps evaluates one
+// shell quartet, with the class's angular momenta as compile-time parameters.
+// Every class has a pair with an f shell; that pair (the larger one where
+// both have) gives the rows: a lane owns one component (a, b) of it and holds
+// that row's integrals over all components (c, d) of the other pair in
+// registers.  Units of work are (primitive quartet, root):
+//   1. one thread per (unit, axis): root and weight from the 7-root table, the
+//      2D vertical recurrence and the transfer to shell B in registers, the
+//      result h[a][b][f], f <= lc+ld, to shared memory;
+//   2. every row lane reads its three h rows, transfers them to (c, d) in
+//      registers and adds the products: two FMAs an integral and root and
+//      3 (lc+ld+1) shared loads a root, where one thread per component read
+//      three tables an integral and root.
+// Digestion (DIRFCK rules, src/rhf/rys/int3011_rysgen.F90 digestion) runs on
+// the same registers: a lane forms its sums for all six updates, those that
+// several rows share are added up over the group (shuffles for the ket pair's
+// J, shared memory for the K rows), and one FP64 atomic per function pair goes
+// to F, about one for eight integrals instead of six each.  The six atomics
+// an integral (4e9 a build of a 30-atom cluster, 187 G/s) and the tables' shared
+// loads bounded the earlier form.  FP64 only: a mixed-precision build runs its
+// f classes in FP64.
 #include "quartet.cuh"
 
 namespace liberi {
 
-constexpr int FCLASS_THREADS = 128;
-
-// Shared-memory bytes of one group of a class: the quartet's block, npq
-// rounds' VRR and 2D-integral tables, the component index tables.
 __host__ __device__ constexpr int fnc(int l) { return (l + 1) * (l + 2) / 2; }
-__host__ __device__ constexpr size_t fgroup_bytes(int la, int lb, int lc, int ld, int npq) {
-    return sizeof(double) * ((size_t)fnc(la) * fnc(lb) * fnc(lc) * fnc(ld) +
-                             (size_t)npq * 3 * ((la + lb + lc + ld) / 2 + 1) *
-                                 ((la + lb + 1) * (lc + ld + 1) + (la + 1) * (lb + 1) * (lc + 1) * (ld + 1))) +
-           3 * (size_t)(fnc(la) * fnc(lb) + fnc(lc) * fnc(ld)) + 16;
-}
-// One warp per quartet where the working set of one primitive quartet per
-// round fits 24 KB, else the whole CTA.
-__host__ __device__ constexpr bool fwarp_mode(int la, int lb, int lc, int ld) {
-    return fgroup_bytes(la, lb, lc, ld, 1) <= 24 * 1024;
-}
-// Primitive quartets per round: as many as the group's threads take in step 1
-// (3 n each) within 12 KB per warp group (four CTAs of four warps per SM) or
-// 48 KB per CTA group (four or more CTAs of eight warps per SM where the
-// block allows: a round rarely fills many slots, uncontracted polarisation
-// shells having one primitive each).
-__host__ __device__ constexpr int fnpq(int la, int lb, int lc, int ld, int nt) {
-    int npq = nt / (3 * ((la + lb + lc + ld) / 2 + 1));
-    while (npq > 1 && fgroup_bytes(la, lb, lc, ld, npq) > (nt == 32 ? 12 * 1024 : 48 * 1024)) npq--;
-    return npq < 1 ? 1 : npq;
-}
 
-// Compile-time shape of one class (engine orientation, la >= lb, lc >= ld) for
-// groups of NT threads: one warp (CTAs of four warps) or a whole CTA of NT.
-template <int LA, int LB, int LC, int LD, int NT>
-struct FS {
-    static constexpr int la = LA, lb = LB, lc = LC, ld = LD, nt = NT;
-    static constexpr int block = NT == 32 ? FCLASS_THREADS : NT;
-    static constexpr int nroot = (LA + LB + LC + LD) / 2 + 1;
-    static constexpr int nb = fnc(LB), nc = fnc(LC), nd = fnc(LD);
-    static constexpr int ncd = nc * nd, ncomp = fnc(LA) * nb * ncd;
-    static constexpr int e1 = LA + LB + 1, f1 = LC + LD + 1;              // VRR extents
-    static constexpr int nab2 = (LA + 1) * (LB + 1), ncd2 = (LC + 1) * (LD + 1);  // 2D index extents
-    static constexpr int npq = fnpq(LA, LB, LC, LD, NT);
-    static constexpr int group_doubles = (int)((fgroup_bytes(LA, LB, LC, LD, npq) + 15) / 16 * 2);
+// Shape of one class: rows (f, LB), kets (LC, LD).
+//   SL  a ten-row class puts three slots of rows into a warp, each taking
+//       every third unit
+//   KS  a ket pair of more than 60 components ((ff|ff) alone) is split over
+//       two sets of row lanes, so that a lane's block stays in registers
+template <int LB_, int LC_, int LD_>
+struct FR {
+    static constexpr int LB = LB_, LC = LC_, LD = LD_;
+    static constexpr int NB = fnc(LB), NC = fnc(LC), ND = fnc(LD), NROW = 10 * NB;
+    static constexpr int NR = (3 + LB + LC + LD) / 2 + 1;
+    static constexpr int F1 = LC + LD + 1, F1P = F1 | 1;  // odd row stride: no bank conflicts
+    static constexpr int KS = NC * ND > 60 ? 2 : 1, NCS = NC / KS;
+    static constexpr int SL = NROW == 10 ? 3 : 1;
+    static constexpr int RT = (NROW + 31) / 32 * 32;  // row lanes of one split
+    static constexpr int GT = RT * KS;                // threads per quartet
+    static constexpr int BLOCK = GT == 32 ? 128 : GT, GROUPS = BLOCK / GT;
+    static constexpr int UNIT = 3 * 4 * (LB + 1) * F1P;  // doubles of one unit's h rows
+    static constexpr int UFIT = (GT == 32 ? 1280 : 5120) / UNIT;  // 10 KB a warp group, 40 KB a CTA group
+    static constexpr int U = UFIT < 1 ? 1 : (UFIT < GT / 3 ? UFIT : GT / 3);  // units per round
+    static constexpr int NK = 2 * (NCS + ND);            // K sums of a row
+    static constexpr int KBUF = KS * NK * NROW;
+    static constexpr int SMEM = U * UNIT > KBUF ? U * UNIT : KBUF;  // doubles per group
+    // resident CTAs from what a lane holds: its block and two of the three 2D
+    // tables, or the vertical recurrence of step 1
+    static constexpr int HOLD_B = NCS * ND + 2 * (LC + 1) * (LD + 1), HOLD_A = (4 + LB) * F1;
+    static constexpr int REGS_ = 2 * (HOLD_A > HOLD_B ? HOLD_A : HOLD_B) + 72;
+    static constexpr int REGS = REGS_ > 255 ? 255 : REGS_;
+    static constexpr int MINB_ = 65536 / (REGS * BLOCK);
+    static constexpr int MINB = MINB_ < 1 ? 1 : MINB_;
 };
 
 namespace {
@@ -78,32 +70,34 @@ __constant__ unsigned char c_cart[4][10][3] = {
     {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}},
     {{2, 0, 0}, {0, 2, 0}, {0, 0, 2}, {1, 1, 0}, {1, 0, 1}, {0, 1, 1}},
     {{3, 0, 0}, {0, 3, 0}, {0, 0, 3}, {2, 1, 0}, {2, 0, 1}, {1, 2, 0}, {0, 2, 1}, {1, 0, 2}, {0, 1, 2}, {1, 1, 1}}};
-__device__ __forceinline__ void cart3(int l, int i, int &x, int &y, int &z) {
-    x = c_cart[l][i][0];
-    y = c_cart[l][i][1];
-    z = c_cart[l][i][2];
+// the same as compile-time tables (digits x y of the f components)
+__host__ __device__ constexpr int fx3(int i) {
+    return i == 0 ? 3 : (i == 3 || i == 4) ? 2 : (i == 5 || i == 7 || i == 9) ? 1 : 0;
 }
+__host__ __device__ constexpr int fy3(int i) {
+    return i == 1 ? 3 : (i == 5 || i == 6) ? 2 : (i == 3 || i == 8 || i == 9) ? 1 : 0;
+}
+__host__ __device__ constexpr int fcx(int l, int i) { return l == 3 ? fx3(i) : cxp(l, i); }
+__host__ __device__ constexpr int fcy(int l, int i) { return l == 3 ? fy3(i) : cyp(l, i); }
+__host__ __device__ constexpr int fcz(int l, int i) { return l - fcx(l, i) - fcy(l, i); }
 
 // per-component normalisation relative to the axial component: sqrt3 on the
 // mixed d, sqrt5 on the six mixed f and sqrt15 on xyz (int3011_rysgen.F90 d03bra)
-__device__ __forceinline__ double cnorm(int l, int i) {
-    if (l == 2) return i >= 3 ? 1.7320508075688772935 : 1.0;
-    if (l == 3) return i == 9 ? 3.8729833462074168852 : (i >= 3 ? 2.2360679774997896964 : 1.0);
-    return 1.0;
+__host__ __device__ constexpr double cnorm(int l, int i) {
+    return l == 2 ? (i >= 3 ? 1.7320508075688772935 : 1.0)
+         : l == 3 ? (i == 9 ? 3.8729833462074168852 : (i >= 3 ? 2.2360679774997896964 : 1.0))
+                  : 1.0;
 }
 
-__device__ __forceinline__ unsigned ftri(unsigned i, unsigned j) {
-    return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i;
-}
-
-// root r and weight of the n-root Rys rule at T (large-T limit above thr,
+// root r and weight of the N-root Rys rule at T (large-T limit above thr,
 // strict: T > thr, else T >= thr; always at and above the table's end)
-__device__ __forceinline__ void rys7_root(int n, int r, double T, double thr, bool strict, const double *tab,
-                                          double &u, double &w) {
+template <int N>
+__device__ __forceinline__ void rys7_root(int r, double T, double thr, bool strict, const double *tab, double &u,
+                                          double &w) {
     const bool asym = (strict ? (T > thr) : (T >= thr)) || T >= RYS7_TMAX;
     if (asym) {
         const double it = 1.0 / T;
-        const double *hr = tab + rys7_herm_off(n);
+        const double *hr = tab + rys7_herm_off(N);
         u = __ldg(hr + r) * it;
         w = __ldg(hr + MAXROOT7 + r) * sqrt(it);
         return;
@@ -111,296 +105,401 @@ __device__ __forceinline__ void rys7_root(int n, int r, double T, double thr, bo
     const double t4 = T * (double)RYS_PER_UNIT;
     const int k = (int)t4;
     const double x = 2.0 * (t4 - (double)k) - 1.0, x2 = x * x, x4 = x2 * x2;
-    const double *base = tab + rys7_table_off(n) + (size_t)k * (2 * n * RYS_NCOEF);
+    const double *base = tab + rys7_table_off(N) + (size_t)k * (2 * N * RYS_NCOEF) + r * RYS_NCOEF;
     double v[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const double *c = base + (h ? n + r : r) * RYS_NCOEF;
-        const double a0 = fma(__ldg(c + 1), x, __ldg(c + 0)), a1 = fma(__ldg(c + 3), x, __ldg(c + 2));
-        const double a2 = fma(__ldg(c + 5), x, __ldg(c + 4)), a3 = fma(__ldg(c + 7), x, __ldg(c + 6));
+        double c0, c1, c2, c3, c4, c5, c6, c7;
+        ldg_v4f64(base + h * (N * RYS_NCOEF), c0, c1, c2, c3);
+        ldg_v4f64(base + h * (N * RYS_NCOEF) + 4, c4, c5, c6, c7);
+        const double a0 = fma(c1, x, c0), a1 = fma(c3, x, c2);
+        const double a2 = fma(c5, x, c4), a3 = fma(c7, x, c6);
         v[h] = fma(fma(a3, x2, a2), x4, fma(a1, x2, a0));
     }
     u = v[0];
     w = v[1];
 }
 
-}  // namespace
-
-// A group of NT threads evaluates one quartet at a time: a whole CTA (NT = 128)
-// for the classes with large blocks, one warp (NT = 32) for the others, four
-// warps of a CTA then working on four tasks with their own shared memory and
-// warp barriers only.
-template <int NT>
-__device__ __forceinline__ int group_rank() { return NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x; }
-template <int NT>
+template <int GT>
 __device__ __forceinline__ void group_sync() {
-    if constexpr (NT == 32) __syncwarp();
+    if constexpr (GT == 32) __syncwarp();
     else __syncthreads();
 }
 
-// Shared-memory layout of one group: the quartet's block, the VRR tables and
-// the 2D-integral tables of a round, and per component the 2D index on each axis.
-struct FSmem {
-    double *acc;         // [ncomp]
-    double *g;           // [npq][3n][e1*f1]
-    double *G;           // [npq][3n][nab2*ncd2]
-    unsigned char *gab;  // [3][na*nb]: a*(lb+1)+b per axis
-    unsigned char *gcd;  // [3][ncd]: c*(ld+1)+d per axis
-    int nab;
+// The shell quartet of pairs P (rows) and Q (kets).
+struct FQuartet {
+    double4 A, C;
+    double AB[3], CD[3];
+    int p0, np, q0, nq;
+};
+__device__ __forceinline__ FQuartet fquartet(const DevBasis &b, int P, int Q) {
+    FQuartet f;
+    const int2 sab = b.pair_shell[P], scd = b.pair_shell[Q];
+    f.A = b.shell_xyz[sab.x];
+    f.C = b.shell_xyz[scd.x];
+    const double4 B = b.shell_xyz[sab.y], D = b.shell_xyz[scd.y];
+    f.AB[0] = f.A.x - B.x, f.AB[1] = f.A.y - B.y, f.AB[2] = f.A.z - B.z;
+    f.CD[0] = f.C.x - D.x, f.CD[1] = f.C.y - D.y, f.CD[2] = f.C.z - D.z;
+    f.p0 = b.pair_prim0[P], f.np = b.pair_nprim[P];
+    f.q0 = b.pair_prim0[Q], f.nq = b.pair_nprim[Q];
+    return f;
+}
+
+// Step 1 for one (unit, axis): h[a][b][f] to hs (rows of F1P doubles).
+template <typename S>
+__device__ __forceinline__ void fstage(const DevBasis &b, const FQuartet &f, int unit, int x, double thr, bool strict,
+                                       const double *__restrict__ tab7, double *hs) {
+    constexpr int LB = S::LB, F1 = S::F1, E1 = 4 + LB;
+    const int pq = unit / S::NR, r = unit - pq * S::NR;
+    const int ip = pq / f.nq, iq = pq - ip * f.nq;
+    const double4 Pp = ldg_double4(b.prim_P + f.p0 + ip), Qp = ldg_double4(b.prim_P + f.q0 + iq);
+    const double2 Xp = b.prim_X[f.p0 + ip], Xq = b.prim_X[f.q0 + iq];
+    const double p = Pp.w, q = Qp.w, rs = rsqrt(p + q), ipq = rs * rs;
+    const double dx = Pp.x - Qp.x, dy = Pp.y - Qp.y, dz = Pp.z - Qp.z;
+    const double T = p * q * ipq * (dx * dx + dy * dy + dz * dz);
+    double u, w;
+    rys7_root<S::NR>(r, T, thr, strict, tab7, u, w);
+    u *= ipq;
+    const double fq = q * u, fp = p * u;
+    const double PA = x == 0 ? Pp.x - f.A.x : (x == 1 ? Pp.y - f.A.y : Pp.z - f.A.z);
+    const double QC = x == 0 ? Qp.x - f.C.x : (x == 1 ? Qp.y - f.C.y : Qp.z - f.C.z);
+    const double PQ = x == 0 ? dx : (x == 1 ? dy : dz);
+    const double ab = x == 0 ? f.AB[0] : (x == 1 ? f.AB[1] : f.AB[2]);
+    double g[E1][F1];
+    vrr<E1 - 1, F1 - 1, double>(g, PA - fq * PQ, QC + fp * PQ, Xp.y * (1.0 - fq), Xq.y * (1.0 - fp), 0.5 * u,
+                                x == 0 ? Xp.x * Xq.x * rs * w : 1.0);
+#pragma unroll
+    for (int k = 0; k < F1; k++) {
+        double t[E1];
+#pragma unroll
+        for (int e = 0; e < E1; e++) t[e] = g[e][k];
+#pragma unroll
+        for (int bb = 0; bb <= LB; bb++) {
+#pragma unroll
+            for (int a = 0; a < 4; a++) hs[(a * (LB + 1) + bb) * S::F1P + k] = t[a];
+#pragma unroll
+            for (int e = 0; e + 1 < E1 - bb; e++) t[e] = fma(ab, t[e], t[e + 1]);
+        }
+    }
+}
+
+// the 2D integrals of one axis over (c, d) from a row of h
+template <typename S>
+__device__ __forceinline__ void fket(const double *hs, double cd, double (&I)[S::LC + 1][S::LD + 1]) {
+    double t[S::F1];
+#pragma unroll
+    for (int k = 0; k < S::F1; k++) t[k] = hs[k];
+#pragma unroll
+    for (int d = 0; d <= S::LD; d++) {
+#pragma unroll
+        for (int c = 0; c <= S::LC; c++) I[c][d] = t[c];
+#pragma unroll
+        for (int k = 0; k + 1 < S::F1 - d; k++) t[k] = fma(cd, t[k], t[k + 1]);
+    }
+}
+
+// Step 2 for one unit: the row's products for components C of split H.
+template <typename S, int H>
+__device__ __forceinline__ void fassemble(const double *h, int ox, int oy, int oz, const double (&CD)[3],
+                                          double (&acc)[S::NCS][S::ND]) {
+    constexpr int PL = S::UNIT / 3;
+    double ix[S::LC + 1][S::LD + 1], iy[S::LC + 1][S::LD + 1], iz[S::LC + 1][S::LD + 1];
+    fket<S>(h + ox, CD[0], ix);
+    fket<S>(h + PL + oy, CD[1], iy);
+    fket<S>(h + 2 * PL + oz, CD[2], iz);
+#pragma unroll
+    for (int c = 0; c < S::NCS; c++)
+#pragma unroll
+        for (int d = 0; d < S::ND; d++) {
+            const int ic = H * S::NCS + c;
+            acc[c][d] = fma(ix[fcx(S::LC, ic)][fcx(S::LD, d)] * iy[fcy(S::LC, ic)][fcy(S::LD, d)],
+                            iz[fcz(S::LC, ic)][fcz(S::LD, d)], acc[c][d]);
+        }
+}
+
+struct FShells {
+    int bfA, bfB, bfC, bfD;
+    bool iandj, kandl, same;
 };
 
-// Carves the layout, fills the index tables and zeroes the block (the caller
-// synchronises the group before use).
+// unique-component loops and 0.5 factors (0: skipped) of coinciding shells
 template <typename S>
-__device__ __forceinline__ FSmem fsmem_setup(const S &s, double *fsm) {
-    constexpr int NT = S::nt;
-    FSmem m;
-    const int tid = group_rank<NT>(), nrx = 3 * s.nroot;
-    m.acc = fsm;
-    m.g = m.acc + s.ncomp;
-    m.G = m.g + (size_t)s.npq * nrx * s.e1 * s.f1;
-    m.gab = reinterpret_cast<unsigned char *>(m.G + (size_t)s.npq * nrx * s.nab2 * s.ncd2);
-    m.nab = s.ncomp / s.ncd;
-    m.gcd = m.gab + 3 * m.nab;
-    for (int i = tid; i < m.nab; i += NT) {
-        int ax, ay, az, bx, by, bz;
-        cart3(s.la, i / s.nb, ax, ay, az);
-        cart3(s.lb, i % s.nb, bx, by, bz);
-        m.gab[i] = (unsigned char)(ax * (s.lb + 1) + bx);
-        m.gab[m.nab + i] = (unsigned char)(ay * (s.lb + 1) + by);
-        m.gab[2 * m.nab + i] = (unsigned char)(az * (s.lb + 1) + bz);
+__device__ __forceinline__ double ffactor(const FShells &s, int ia, int ib, int ic, int id) {
+    if (S::LB == 3 && s.iandj && ib > ia) return 0.0;
+    if (S::LC == S::LD && s.kandl && id > ic) return 0.0;
+    if (S::LC == 3 && S::LD == S::LB && s.same) {
+        const int pij = s.iandj ? ia * (ia + 1) / 2 + ib : ia * S::NB + ib;
+        const int pkl = s.kandl ? ic * (ic + 1) / 2 + id : ic * S::ND + id;
+        if (pkl > pij) return 0.0;
     }
-    for (int i = tid; i < s.ncd; i += NT) {
-        int cx, cy, cz, dx, dy, dz;
-        cart3(s.lc, i / s.nd, cx, cy, cz);
-        cart3(s.ld, i % s.nd, dx, dy, dz);
-        m.gcd[i] = (unsigned char)(cx * (s.ld + 1) + dx);
-        m.gcd[s.ncd + i] = (unsigned char)(cy * (s.ld + 1) + dy);
-        m.gcd[2 * s.ncd + i] = (unsigned char)(cz * (s.ld + 1) + dz);
-    }
-    for (int c = tid; c < s.ncomp; c += NT) m.acc[c] = 0.0;
-    return m;
+    const int mu = s.bfA + ia, nu = s.bfB + ib, la = s.bfC + ic, si = s.bfD + id;
+    double f = 1.0;
+    if (mu == nu) f *= 0.5;
+    if (la == si) f *= 0.5;
+    if ((mu == la && nu == si) || (mu == si && nu == la)) f *= 0.5;
+    return f;
 }
 
-// Adds the contracted block of the quartet (P|Q) (pair P = (A,B), Q = (C,D))
-// to m.acc: every thread keeps its own components c = rank + k * NT.  Called
-// by the whole group; every round of primitive quartets ends with a group
-// barrier, so the tables may be reused on return.
-template <typename S>
-__device__ __forceinline__ void fquartet_block(const S &s, const FSmem &m, const DevBasis &b, int P, int Q,
-                                               double thr, bool strict, const double *__restrict__ tab7) {
-    constexpr int NT = S::nt;
-    const int tid = group_rank<NT>();
-    const int n = s.nroot, nrx = 3 * n;
-    const int gsz = s.e1 * s.f1;      // one VRR table
-    const int Gsz = s.nab2 * s.ncd2;  // one 2D-integral table
-    double *g = m.g, *G = m.G;
-    const int nab = m.nab;
-    const unsigned char *gab = m.gab, *gcd = m.gcd;
-    const int2 sab = b.pair_shell[P], scd = b.pair_shell[Q];
-    const double4 A = b.shell_xyz[sab.x], B = b.shell_xyz[sab.y];
-    const double4 C = b.shell_xyz[scd.x], D = b.shell_xyz[scd.y];
-    const int p0 = b.pair_prim0[P], np = b.pair_nprim[P];
-    const int q0 = b.pair_prim0[Q], nq = b.pair_nprim[Q];
-    const double AB[3] = {A.x - B.x, A.y - B.y, A.z - B.z};
-    const double CD[3] = {C.x - D.x, C.y - D.y, C.z - D.z};
-    const int npq_total = np * nq;
-    for (int pq0 = 0; pq0 < npq_total; pq0 += s.npq) {
-        // slots of this round that hold a primitive quartet (uncontracted
-        // polarisation shells leave most of them empty): steps 2 and 3 cover
-        // only these
-        const int nslot = min(s.npq, npq_total - pq0);
-        // 1. roots and the vertical recurrence, one thread per (slot, root, axis)
-        if (tid < nslot * nrx) {
-            const int slot = tid / nrx, rx = tid - slot * nrx;
-            const int r = rx / 3, x = rx - 3 * r;
-            const int pq = pq0 + slot;
-            double *gs = g + (size_t)(slot * nrx + rx) * gsz;
-            if (pq < npq_total) {
-                const int ip = pq / nq, iq = pq - ip * nq;
-                const double4 Pp = b.prim_P[p0 + ip], Qp = b.prim_P[q0 + iq];
-                const double2 Xp = b.prim_X[p0 + ip], Xq = b.prim_X[q0 + iq];
-                const double p = Pp.w, q = Qp.w, ipq = 1.0 / (p + q);
-                const double dx = Pp.x - Qp.x, dy = Pp.y - Qp.y, dz = Pp.z - Qp.z;
-                const double T = p * q * ipq * (dx * dx + dy * dy + dz * dz);
-                double u, w;
-                rys7_root(n, r, T, thr, strict, tab7, u, w);
-                const double B00 = 0.5 * u * ipq;
-                const double B10 = 0.5 / p * (1.0 - q * u * ipq);
-                const double B01 = 0.5 / q * (1.0 - p * u * ipq);
-                const double PA = x == 0 ? Pp.x - A.x : (x == 1 ? Pp.y - A.y : Pp.z - A.z);
-                const double QC = x == 0 ? Qp.x - C.x : (x == 1 ? Qp.y - C.y : Qp.z - C.z);
-                const double PQ = x == 0 ? dx : (x == 1 ? dy : dz);
-                const double C00 = PA - q * u * ipq * PQ;
-                const double Cp00 = QC + p * u * ipq * PQ;
-                const double g00 = x == 0 ? Xp.x * Xq.x * sqrt(ipq) * w : 1.0;
-                const int e1 = s.e1, f1 = s.f1;
-                gs[0] = g00;
-                for (int e = 0; e + 1 < e1; e++) {
-                    double v = C00 * gs[e * f1];
-                    if (e > 0) v += (double)e * B10 * gs[(e - 1) * f1];
-                    gs[(e + 1) * f1] = v;
-                }
-                for (int f = 0; f + 1 < f1; f++)
-                    for (int e = 0; e < e1; e++) {
-                        double v = Cp00 * gs[e * f1 + f];
-                        if (f > 0) v += (double)f * B01 * gs[e * f1 + f - 1];
-                        if (e > 0) v += (double)e * B00 * gs[(e - 1) * f1 + f];
-                        gs[e * f1 + f + 1] = v;
-                    }
-            }
+__device__ __forceinline__ void fadd(double *F, unsigned i, unsigned j, double v) {
+    if (v != 0.0) atomicAdd(F + tri0(i, j), v);
+}
+
+// Sums v[0..N-1] over the warp; the total of value i arrives at lane i (mod
+// the padded length).  31 exchanges for 32 values.
+template <int N>
+__device__ __forceinline__ double warp_scatter_sum(double (&v)[N], int lane) {
+    static_assert(N <= 32 && (N & (N - 1)) == 0, "padded to a power of two");
+#pragma unroll
+    for (int s = 16; s >= N; s >>= 1)
+#pragma unroll
+        for (int i = 0; i < N; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], s);
+#pragma unroll
+    for (int s = N / 2; s >= 1; s >>= 1)
+#pragma unroll
+        for (int i = 0; i < s; i++) {
+            const bool up = (lane & s) != 0;
+            const double keep = up ? v[i + s] : v[i], send = up ? v[i] : v[i + s];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
         }
-        group_sync<NT>();
-        // 2. transfer to the 2D integrals of every (slot, root, axis)
-        const int nG = nslot * nrx * Gsz;
-        for (int idx = tid; idx < nG; idx += NT) {
-            const int tab_i = idx / Gsz, rem = idx - tab_i * Gsz;
-            const int x = tab_i % 3;
-            const int iab = rem / s.ncd2, icd = rem - iab * s.ncd2;
-            const int ia = iab / (s.lb + 1), ib = iab - ia * (s.lb + 1);
-            const int ic = icd / (s.ld + 1), id = icd - ic * (s.ld + 1);
-            const double ab = AB[x], cd = CD[x];
-            const double *gs = g + (size_t)tab_i * gsz;
-            // i, k from the top: weights C(ib,i) AB^(ib-i) and C(id,k) CD^(id-k),
-            // the binomial updated as C(n,m-1) = C(n,m) m / (n-m+1)
-            double sum = 0.0, wb = 1.0;
-            for (int i = ib; i >= 0; i--) {
-                double inner = 0.0, wd = 1.0;
-                for (int k = id; k >= 0; k--) {
-                    inner = fma(wd, gs[(ia + i) * s.f1 + ic + k], inner);
-                    wd *= cd * (double)k / (double)(id - k + 1);
-                }
-                sum = fma(wb, inner, sum);
-                wb *= ab * (double)i / (double)(ib - i + 1);
-            }
-            G[idx] = sum;
+    return v[0];
+}
+constexpr int fpow2(int x) { return x <= 1 ? 1 : 2 * fpow2((x + 1) / 2); }
+
+// Digestion of a lane's row over split H: the row pair's J at once, the ket
+// pair's J over the warp, the row's K sums to kb[value][row].
+template <typename S, int H>
+__device__ __forceinline__ void fdigest(double (&acc)[S::NCS][S::ND], bool rowok, int row, int lane,
+                                        const FShells &s, const ClassArgs &a, double *kb) {
+    constexpr int NCS = S::NCS, ND = S::ND;
+    const double *__restrict__ Dm = a.Dm, *__restrict__ Dk = a.Dm + a.k_offset;
+    const unsigned n = (unsigned)a.nbf;
+    const bool distinct = !s.iandj && !s.kandl && !s.same;
+    const int ia = rowok ? row / S::NB : 0, ib = rowok ? row % S::NB : 0;
+    const unsigned mu = s.bfA + ia, nu = s.bfB + ib;
+    const double nab = cnorm(3, ia) * cnorm(S::LB, ib);
+    const double dAB = 4.0 * dget(Dm, n, mu, nu);
+    double jab = 0.0, dAD[ND], dBD[ND], kad[ND], kbd[ND];
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        dAD[d] = dget(Dk, n, mu, s.bfD + d);
+        dBD[d] = dget(Dk, n, nu, s.bfD + d);
+        kad[d] = kbd[d] = 0.0;
+    }
+#pragma unroll
+    for (int c = 0; c < NCS; c++) {
+        const int ic = H * NCS + c;
+        const double dAC = dget(Dk, n, mu, s.bfC + ic), dBC = dget(Dk, n, nu, s.bfC + ic);
+        double kac = 0.0, kbc = 0.0;
+#pragma unroll
+        for (int d = 0; d < ND; d++) {
+            double v = acc[c][d] * (nab * (cnorm(S::LC, ic) * cnorm(S::LD, d)));
+            v = !rowok || fabs(v) < a.cut ? 0.0 : v;
+            if (!distinct) v *= ffactor<S>(s, ia, ib, ic, d);
+            jab = fma(v, dget(Dm, n, s.bfC + ic, s.bfD + d), jab);
+            kac = fma(v, dBD[d], kac);
+            kad[d] = fma(v, dBC, kad[d]);
+            kbc = fma(v, dAD[d], kbc);
+            kbd[d] = fma(v, dAC, kbd[d]);
+            acc[c][d] = v * dAB;
         }
-        group_sync<NT>();
-        // 3. assembly: every thread its own components
-        for (int c = tid; c < s.ncomp; c += NT) {
-            const int iab = c / s.ncd, icd = c - iab * s.ncd;
-            const int ix = gab[iab] * s.ncd2 + gcd[icd];
-            const int iy = gab[nab + iab] * s.ncd2 + gcd[s.ncd + icd];
-            const int iz = gab[2 * nab + iab] * s.ncd2 + gcd[2 * s.ncd + icd];
-            double v = 0.0;
-            const int ntab = nslot * n;
-            for (int tr = 0; tr < ntab; tr++) {
-                const double *Gt = G + (size_t)tr * 3 * Gsz;
-                v = fma(Gt[ix] * Gt[Gsz + iy], Gt[2 * Gsz + iz], v);
-            }
-            m.acc[c] += v;
+        if (rowok) {
+            kb[c * S::NROW + row] = kac;
+            kb[(NCS + ND + c) * S::NROW + row] = kbc;
         }
-        group_sync<NT>();
+    }
+    if (rowok) {
+#pragma unroll
+        for (int d = 0; d < ND; d++) {
+            kb[(NCS + d) * S::NROW + row] = kad[d];
+            kb[(2 * NCS + ND + d) * S::NROW + row] = kbd[d];
+        }
+        fadd(a.F, mu, nu, 4.0 * jab);
+    }
+    constexpr int NV = NCS * ND;
+#pragma unroll
+    for (int v0 = 0; v0 < NV; v0 += 32) {
+        constexpr int W = NV >= 32 ? 32 : fpow2(NV);
+        double v[W];
+#pragma unroll
+        for (int i = 0; i < W; i++) v[i] = v0 + i < NV ? acc[(v0 + i) / ND][(v0 + i) % ND] : 0.0;
+        const double t = warp_scatter_sum<W>(v, lane);
+        const int i = v0 + lane;
+        if (lane < W && i < NV) fadd(a.F, s.bfC + H * NCS + i / ND, s.bfD + i % ND, t);
     }
 }
 
-// NT = 256: one task per CTA; NT = 32: one task per warp (four per CTA).
-template <typename S>
-__global__ void __launch_bounds__(S::block) fclass_kernel(ClassArgs a, const double *__restrict__ tab7) {
-    constexpr int NT = S::nt;
-    constexpr S s{};
-    constexpr int GROUPS = S::block / NT;
-    const int grp = NT == 32 ? (int)(threadIdx.x >> 5) : 0;
-    const int task = (int)blockIdx.x * GROUPS + grp;
-    if (task >= a.ntasks) return;  // the whole group (only warp barriers follow in warp mode)
+}  // namespace
+
+// SWAP: the class's ket pair holds the f shell and gives the rows.
+template <typename S, bool SWAP>
+__global__ void __launch_bounds__(S::BLOCK, S::MINB) fclass_kernel(ClassArgs a, const double *__restrict__ tab7) {
+    constexpr int GT = S::GT, NROW = S::NROW;
+    const int grp = S::GROUPS > 1 ? (int)(threadIdx.x >> 5) : 0;
+    const int task = (int)blockIdx.x * S::GROUPS + grp;
+    if (task >= a.ntasks) return;  // the whole group (only warp barriers follow where a CTA holds several)
     extern __shared__ __align__(16) double fsm[];
-    const int tid = group_rank<NT>();
-    const FSmem m = fsmem_setup(s, fsm + (size_t)grp * s.group_doubles);
-    double *acc = m.acc;
-    group_sync<NT>();
-
+    double *sm = fsm + (size_t)grp * S::SMEM;
+    const int tid = S::GROUPS > 1 ? (int)(threadIdx.x & 31) : (int)threadIdx.x, lane = tid & 31;
+    const int half = S::KS > 1 ? tid / S::RT : 0, rt = tid - half * S::RT;
+    const int slot = S::SL > 1 ? rt / NROW : 0, row = S::SL > 1 ? rt % NROW : rt;
+    const bool rowok = S::SL > 1 ? rt < S::SL * NROW : rt < NROW;
+    const int ia = rowok ? row / S::NB : 0, ib = rowok ? row % S::NB : 0;
+    const int ox = (c_cart[3][ia][0] * (S::LB + 1) + c_cart[S::LB][ib][0]) * S::F1P;
+    const int oy = (c_cart[3][ia][1] * (S::LB + 1) + c_cart[S::LB][ib][1]) * S::F1P;
+    const int oz = (c_cart[3][ia][2] * (S::LB + 1) + c_cart[S::LB][ib][2]) * S::F1P;
     const int4 t = a.tasks[task];
     const DevBasis &b = a.b;
-    const int P = a.bra_ids[t.x];
-    const int2 sab = b.pair_shell[P];
-    const int bfA = b.shell_bf0[sab.x], bfB = b.shell_bf0[sab.y];
-    const unsigned nbf = (unsigned)a.nbf;
-    const double *Dm = a.Dm, *Dk = a.Dm + a.k_offset;
 
     for (int qi = 0; qi < t.z; qi++) {
         const int j = t.y + qi;
         if (a.rs.nsize > 1 && !quartet_owned(a, t.x, j)) continue;  // uniform over the group
-        const int Q = a.ket_ids[j];
-        const int2 scd = b.pair_shell[Q];
-        const int bfC = b.shell_bf0[scd.x], bfD = b.shell_bf0[scd.y];
-        fquartet_block(s, m, b, P, Q, a.thr, a.strict, tab7);
-        // digestion of this thread's components (the same components it
-        // accumulated: no barrier needed before the reads)
-        const bool iandj = sab.x == sab.y, kandl = scd.x == scd.y;
-        const bool same = sab.x == scd.x && sab.y == scd.y;
-        for (int c = tid; c < s.ncomp; c += NT) {
-            double val = acc[c];
-            acc[c] = 0.0;
-            const int iab = c / s.ncd, icd = c - iab * s.ncd;
-            const int ia = iab / s.nb, ib = iab - ia * s.nb;
-            const int ic = icd / s.nd, id = icd - ic * s.nd;
-            if (iandj && ib > ia) continue;
-            if (kandl && id > ic) continue;
-            if (same) {
-                const int pij = iandj ? ia * (ia + 1) / 2 + ib : ia * s.nb + ib;
-                const int pkl = kandl ? ic * (ic + 1) / 2 + id : ic * s.nd + id;
-                if (pkl > pij) continue;
+        const int pb = a.bra_ids[t.x], pk = a.ket_ids[j];
+        const int P = SWAP ? pk : pb, Q = SWAP ? pb : pk;
+        const FQuartet f = fquartet(b, P, Q);
+        double acc[S::NCS][S::ND];
+#pragma unroll
+        for (int c = 0; c < S::NCS; c++)
+#pragma unroll
+            for (int d = 0; d < S::ND; d++) acc[c][d] = 0.0;
+        const int nunit = f.np * f.nq * S::NR;
+#pragma unroll 1
+        for (int u0 = 0; u0 < nunit; u0 += S::U) {
+            const int nu = min(S::U, nunit - u0);
+            if (tid < 3 * nu) {
+                const int uu = tid / 3, x = tid - 3 * uu;
+                fstage<S>(b, f, u0 + uu, x, a.thr, a.strict, tab7, sm + uu * S::UNIT + x * (S::UNIT / 3));
             }
-            val *= cnorm(s.la, ia) * cnorm(s.lb, ib) * cnorm(s.lc, ic) * cnorm(s.ld, id);
-            if (fabs(val) < a.cut) continue;
-            unsigned i2 = bfA + ia, j2 = bfB + ib, k2 = bfC + ic, l2 = bfD + id;
-            if (i2 < j2) { const unsigned tt = i2; i2 = j2; j2 = tt; }
-            if (k2 < l2) { const unsigned tt = k2; k2 = l2; l2 = tt; }
-            unsigned ii = i2, jj = j2, kk = k2, ll = l2;
-            if (ii < kk || (ii == kk && jj < ll)) { ii = k2; jj = l2; kk = i2; ll = j2; }
-            if (ii == jj) val *= 0.5;
-            if (kk == ll) val *= 0.5;
-            if (ii == kk && jj == ll) val *= 0.5;
-            const double v4 = 4.0 * val;
-            atomicAdd(a.F + ftri(ii, jj), v4 * Dm[kk * nbf + ll]);
-            atomicAdd(a.F + ftri(kk, ll), v4 * Dm[ii * nbf + jj]);
-            atomicAdd(a.F + ftri(ii, kk), -val * Dk[jj * nbf + ll]);
-            atomicAdd(a.F + ftri(jj, ll), -val * Dk[ii * nbf + kk]);
-            atomicAdd(a.F + ftri(ii, ll), -val * Dk[jj * nbf + kk]);
-            atomicAdd(a.F + ftri(jj, kk), -val * Dk[ii * nbf + ll]);
+            group_sync<GT>();
+            if (rowok) {
+#pragma unroll 1
+                for (int u = slot; u < nu; u += S::SL) {
+                    const double *h = sm + u * S::UNIT;
+                    if (S::KS == 1 || half == 0) fassemble<S, 0>(h, ox, oy, oz, f.CD, acc);
+                    else fassemble<S, S::KS - 1>(h, ox, oy, oz, f.CD, acc);
+                }
+            }
+            group_sync<GT>();
         }
+        if constexpr (S::SL > 1) {  // the slots' partial rows
+            static_assert(S::SL == 3, "lanes row, row + NROW, row + 2 NROW");
+#pragma unroll
+            for (int c = 0; c < S::NCS; c++)
+#pragma unroll
+                for (int d = 0; d < S::ND; d++) {
+                    const double v = acc[c][d];
+                    acc[c][d] = v + __shfl_down_sync(0xffffffffu, v, NROW) + __shfl_down_sync(0xffffffffu, v, 2 * NROW);
+                }
+        }
+        const int2 sab = b.pair_shell[P], scd = b.pair_shell[Q];
+        FShells s;
+        s.bfA = b.shell_bf0[sab.x], s.bfB = b.shell_bf0[sab.y];
+        s.bfC = b.shell_bf0[scd.x], s.bfD = b.shell_bf0[scd.y];
+        s.iandj = sab.x == sab.y;
+        s.kandl = scd.x == scd.y;
+        s.same = sab.x == scd.x && sab.y == scd.y;
+        const bool own = rowok && slot == 0;
+        double *kb = sm + half * (S::NK * NROW);
+        if (S::KS == 1 || half == 0) fdigest<S, 0>(acc, own, row, lane, s, a, kb);
+        else fdigest<S, S::KS - 1>(acc, own, row, lane, s, a, kb);
+        group_sync<GT>();
+        // the K sums over B (rows of A) and over A (rows of B)
+        constexpr int NV = S::NCS + S::ND, RT = S::RT;
+        for (int i = rt; i < 10 * NV; i += RT) {
+            const int v = i / 10, r = i - 10 * v;
+            double sum = 0.0;
+            for (int k = 0; k < S::NB; k++) sum += kb[v * NROW + r * S::NB + k];
+            const int col = v < S::NCS ? s.bfC + half * S::NCS + v : s.bfD + v - S::NCS;
+            fadd(a.F, s.bfA + r, col, -sum);
+        }
+        for (int i = rt; i < S::NB * NV; i += RT) {
+            const int v = i / S::NB, r = i - S::NB * v;
+            double sum = 0.0;
+            for (int k = 0; k < 10; k++) sum += kb[(NV + v) * NROW + k * S::NB + r];
+            const int col = v < S::NCS ? s.bfC + half * S::NCS + v : s.bfD + v - S::NCS;
+            fadd(a.F, s.bfB + r, col, -sum);
+        }
+        if (t.z > 1) group_sync<GT>();
     }
 }
 
-// Schwarz values of f pairs: one CTA per pair P of one class, the (P|P) block
-// as in the class kernel, then sqrt(max over components |(ab|ab)|) of the
-// normalised integrals into out[P] (global pair index).
+// Schwarz values of f pairs: one group per pair P of one class, the diagonal
+// (ab|ab) of the (P|P) block (one value a row lane), then sqrt(max over
+// components |(ab|ab)|) of the normalised integrals into out[P].
 template <typename S>
-__global__ void __launch_bounds__(FCLASS_THREADS) fschwarz_kernel(DevBasis b, int pair_off, int npairs,
-                                                                  const double *__restrict__ tab7, double *out) {
-    if ((int)blockIdx.x >= npairs) return;
-    constexpr S s{};
-    static_assert(S::nt == FCLASS_THREADS, "one pair per CTA");
+__global__ void __launch_bounds__(S::BLOCK) fschwarz_kernel(DevBasis b, int pair_off, int npairs,
+                                                            const double *__restrict__ tab7, double *out) {
+    constexpr int GT = S::GT, NROW = S::NROW, PL = S::UNIT / 3;
+    const int grp = S::GROUPS > 1 ? (int)(threadIdx.x >> 5) : 0;
+    const int item = (int)blockIdx.x * S::GROUPS + grp;
+    if (item >= npairs) return;
     extern __shared__ __align__(16) double fsm[];
-    __shared__ double wmax[FCLASS_THREADS / 32];
-    const FSmem m = fsmem_setup(s, fsm);
-    __syncthreads();
-    const int P = pair_off + (int)blockIdx.x;
-    fquartet_block(s, m, b, P, P, RYS7_TMAX, false, tab7);
-    // diagonal components (a b|a b): icd == iab
+    __shared__ double wmax[S::BLOCK / 32];
+    double *sm = fsm + (size_t)grp * S::SMEM;
+    const int tid = S::GROUPS > 1 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
+    // (the ket splits of the block's shape are more slots here)
+    constexpr int SLOTS = S::SL > 1 ? S::SL : S::KS, STRIDE = S::SL > 1 ? NROW : S::RT;
+    const int slot = tid / STRIDE, row = tid % STRIDE;
+    const bool rowok = slot < SLOTS && row < NROW;
+    int e[3][2] = {};
+    if (rowok)
+        for (int x = 0; x < 3; x++) {
+            e[x][0] = c_cart[3][row / S::NB][x];
+            e[x][1] = c_cart[S::LB][row % S::NB][x];
+        }
+    const int P = pair_off + item;
+    const FQuartet f = fquartet(b, P, P);
+    double acc = 0.0;
+    const int nunit = f.np * f.nq * S::NR;
+    for (int u0 = 0; u0 < nunit; u0 += S::U) {
+        const int nu = min(S::U, nunit - u0);
+        if (tid < 3 * nu) {
+            const int uu = tid / 3, x = tid - 3 * uu;
+            fstage<S>(b, f, u0 + uu, x, RYS7_TMAX, false, tab7, sm + uu * S::UNIT + x * PL);
+        }
+        group_sync<GT>();
+        if (rowok)
+            for (int u = slot; u < nu; u += SLOTS) {
+                double prod = 1.0;
+                for (int x = 0; x < 3; x++) {
+                    const double *h = sm + u * S::UNIT + x * PL + (e[x][0] * (S::LB + 1) + e[x][1]) * S::F1P + e[x][0];
+                    double t[4] = {0.0, 0.0, 0.0, 0.0};
+                    for (int k = 0; k <= e[x][1]; k++) t[k] = h[k];
+                    for (int d = e[x][1]; d > 0; d--)
+                        for (int k = 0; k < d; k++) t[k] = fma(f.CD[x], t[k], t[k + 1]);
+                    prod *= t[0];
+                }
+                acc += prod;
+            }
+        group_sync<GT>();
+    }
+    // the slots' partial sums through shared memory, then the maximum
+    if (rowok) sm[slot * NROW + row] = acc;
+    group_sync<GT>();
     double mx = 0.0;
-    for (int iab = threadIdx.x; iab < m.nab; iab += FCLASS_THREADS) {
-        const int ia = iab / s.nb, ib = iab - ia * s.nb;
-        const double nrm = cnorm(s.la, ia) * cnorm(s.lb, ib);
-        mx = fmax(mx, fabs(m.acc[iab * s.ncd + iab]) * nrm * nrm);
+    if (rowok && slot == 0) {
+        for (int k = 1; k < SLOTS; k++) acc += sm[k * NROW + row];
+        const double nrm = cnorm(3, row / S::NB) * cnorm(S::LB, row % S::NB);
+        mx = fabs(acc) * nrm * nrm;
     }
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < FCLASS_THREADS / 32; w++) mx = fmax(mx, wmax[w]);
-        out[P] = sqrt(mx);
+    if constexpr (GT > 32) {
+        if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
+        __syncthreads();
+        for (int w = 0; w < GT / 32; w++) mx = fmax(mx, wmax[w]);
     }
+    if (tid == 0) out[P] = sqrt(mx);
 }
 
 template <int LF>
 static cudaError_t fschwarz_t(int npairs, int pair_off, const DevBasis &b, const double *tab7, double *out,
                               cudaStream_t stream) {
-    using S = FS<3, LF, 3, LF, FCLASS_THREADS>;
-    const size_t smem = (size_t)S::group_doubles * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(fschwarz_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    using S = FR<LF, 3, LF>;
+    const size_t smem = (size_t)S::GROUPS * S::SMEM * sizeof(double);
+    static FuncAttrs attrs;
+    cudaError_t e = attrs.set((const void *)fschwarz_kernel<S>, (int)smem, -1);
     if (e != cudaSuccess) return e;
-    fschwarz_kernel<S><<<(unsigned)npairs, FCLASS_THREADS, smem, stream>>>(b, pair_off, npairs, tab7, out);
+    fschwarz_kernel<S><<<(unsigned)((npairs + S::GROUPS - 1) / S::GROUPS), S::BLOCK, smem, stream>>>(b, pair_off, npairs,
+                                                                                                   tab7, out);
     return cudaGetLastError();
 }
 
@@ -417,17 +516,19 @@ cudaError_t launch_fschwarz(int pair_class, int npairs, int pair_off, const DevB
     }
 }
 
-// one class: warp or CTA groups by its shape, one launch over the plan's tasks
+// one class by its engine orientation (la lb lc ld): the rows are the bra pair
+// where that holds an f shell, else the ket pair
 template <int LA, int LB, int LC, int LD>
 static cudaError_t fclass_t(const ClassArgs &a, const double *tab7, cudaStream_t stream) {
-    constexpr bool W = fwarp_mode(LA, LB, LC, LD);
-    using S = FS<LA, LB, LC, LD, W ? 32 : 2 * FCLASS_THREADS>;
-    constexpr int groups = S::block / S::nt;
-    const size_t smem = (size_t)groups * S::group_doubles * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(fclass_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr bool SWAP = LA < 3;
+    static_assert(SWAP ? LC == 3 : LB >= LD || LC < 3, "rows: the larger f pair");
+    using S = typename std::conditional<SWAP, FR<LD, LA, LB>, FR<LB, LC, LD>>::type;
+    const size_t smem = (size_t)S::GROUPS * S::SMEM * sizeof(double);
+    static FuncAttrs attrs;
+    cudaError_t e = attrs.set((const void *)fclass_kernel<S, SWAP>, (int)smem, -1);
     if (e != cudaSuccess) return e;
-    const unsigned grid = (unsigned)((a.ntasks + groups - 1) / groups);
-    fclass_kernel<S><<<grid, S::block, smem, stream>>>(a, tab7);
+    const unsigned grid = (unsigned)((a.ntasks + S::GROUPS - 1) / S::GROUPS);
+    fclass_kernel<S, SWAP><<<grid, S::BLOCK, smem, stream>>>(a, tab7);
     return cudaGetLastError();
 }
 
