@@ -311,11 +311,20 @@ cudaError_t launch_units(bool low, int ncls, const int *ks, const LaunchCtx &ctx
 // shared-memory evaluation and the 1..7-root table (k_f.cu)
 cudaError_t launch_fschwarz(int pair_class, int npairs, int pair_off, const DevBasis &b, const double *rys_tab7,
                             double *out, cudaStream_t stream);
-cudaError_t launch_schwarz(int pair_class, int npairs, int pair_off, const DevBasis &b,
-                           const double *rys_tab, double *out_per_pair, cudaStream_t stream);
-// per primitive pair of one pair class: sqrt(max |(ab|ab)|) of the primitive alone, rounded up to float
-cudaError_t launch_prim_bound(int pair_class, int npairs, int pair_off, const DevBasis &b, const double *rys_tab,
-                              float *out_per_prim, cudaStream_t stream);
+// Schwarz values of the s/p/d pairs (global pairs class_off[0] .. class_off[NPC_SPD]-1; k_s.cu)
+cudaError_t launch_schwarz(const int *class_off, const DevBasis &b, const double *rys_tab, double *out_per_pair,
+                           cudaStream_t stream);
+// the same straight from the shells (no pair arrays), packed by shells: out[i(i+1)/2 + j], i >= j
+struct ShellTable {
+    const int4 *shell;  // per shell: angular momentum, primitives, first of its exponents and coefficients, -
+    const double4 *xyz;
+    const double *exps, *coefs, *tab;
+    double cux, pref;   // mu R^2 above which a primitive pair is dropped; sqrt(2 pi^(5/2))
+};
+cudaError_t launch_schwarz_shells(const ShellTable &t, int nsh, double *out, cudaStream_t stream);
+// per primitive pair of those pairs: sqrt(max |(ab|ab)|) of the primitive alone, rounded up to float
+cudaError_t launch_prim_bound(const int *class_off, const DevBasis &b, const double *rys_tab, float *out_per_prim,
+                              cudaStream_t stream);
 
 // host-side inputs of the Schwarz generator (host.cpp) and the thread's
 // last-error message, for the allocation-free entry point (noalloc.cu)

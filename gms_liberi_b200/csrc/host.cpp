@@ -792,7 +792,8 @@ static size_t basis_device_bytes(const BasisHost &b, const PairsHost &pr);
 
 static DevBasis dev_basis(liberi_handle h);
 
-static int upload_basis(liberi_handle h, const std::vector<double4> &shell_xyz) {
+// (builds false: a Schwarz table only, without the FP32 tier's data, D and F)
+static int upload_basis(liberi_handle h, const std::vector<double4> &shell_xyz, bool builds = true) {
     const BasisHost &b = h->basis;
     CUDA_TRY(arena_open(h, h->arena_basis, basis_device_bytes(b, h->pairs)));
     ArenaScope scope{h};
@@ -807,12 +808,13 @@ static int upload_basis(liberi_handle h, const std::vector<double4> &shell_xyz) 
     CUDA_TRY(dev_upload(h, &h->dev.prim_X, h->pairs.X.data(), h->pairs.X.size()));
     const std::vector<double> &tab = rys_table_host();
     CUDA_TRY(dev_upload(h, &h->d_tab, tab.data(), tab.size()));
-    const std::vector<float> &tabf = rys_table_f32_host();
-    CUDA_TRY(dev_upload(h, &h->d_tabf, tabf.data(), tabf.size()));
     if (h->pairs.nl[3] > 0) {
         const std::vector<double> &tab7 = rys_table7_host();
         CUDA_TRY(dev_upload(h, &h->d_tab7, tab7.data(), tab7.size()));
     }
+    if (!builds) return LIBERI_OK;
+    const std::vector<float> &tabf = rys_table_f32_host();
+    CUDA_TRY(dev_upload(h, &h->d_tabf, tabf.data(), tabf.size()));
     // Bounds of the single primitive pairs (the FP32 tier's primitive
     // screening), computed on the device from the pair data and tables; then
     // every pair's primitives are put in order of decreasing bound, so that
@@ -824,10 +826,7 @@ static int upload_basis(liberi_handle h, const std::vector<double4> &shell_xyz) 
     std::vector<float> bound(nprim);
     if (nprim) {
         DevBasis db = dev_basis(h);
-        for (int c = 0; c < NPC_SPD; c++) {
-            const int o = pr.class_off[c], n = pr.class_off[c + 1] - o;
-            CUDA_TRY(launch_prim_bound(c, n, o, db, h->d_tab, h->dev.prim_bound, h->stream));
-        }
+        CUDA_TRY(launch_prim_bound(pr.class_off, db, h->d_tab, h->dev.prim_bound, h->stream));
         CUDA_TRY(cudaMemcpyAsync(bound.data(), h->dev.prim_bound, nprim * sizeof(float), cudaMemcpyDeviceToHost,
                                  h->stream));
         CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -2122,6 +2121,45 @@ int liberi_c_quartet_fingerprint(liberi_handle h, uint64_t *out) { return quarte
 
 int liberi_c_quartet_fingerprint_all(liberi_handle h, uint64_t *out) { return quartet_fingerprint(h, NKALL, out); }
 
+// The table of an s/p/d basis from its shells: one allocation, one upload, one
+// launch, the packed table back.
+static int schwarz_shells(liberi_handle h, double *out) {
+    const BasisHost &b = h->basis;
+    const std::vector<double> &tab = rys_table_host();
+    // (exponents and coefficients shell by shell: an s and a p shell may name the same sh_loc)
+    const size_t nsh = (size_t)b.nsh, ntri = nsh * (nsh + 1) / 2;
+    const size_t nex = (size_t)std::accumulate(b.contr_num.begin(), b.contr_num.end(), 0LL);
+    const size_t o_xyz = dev_round(nsh * sizeof(int4)), o_ex = o_xyz + dev_round(nsh * sizeof(double4));
+    const size_t o_co = o_ex + dev_round(nex * sizeof(double)), o_tab = o_co + dev_round(nex * sizeof(double));
+    const size_t o_out = o_tab + dev_round(tab.size() * sizeof(double));
+    std::vector<unsigned char> host(o_out);
+    int4 *shell = reinterpret_cast<int4 *>(host.data());
+    double4 *xyz = reinterpret_cast<double4 *>(host.data() + o_xyz);
+    double *ex = reinterpret_cast<double *>(host.data() + o_ex), *co = reinterpret_cast<double *>(host.data() + o_co);
+    int at = 0;
+    for (int s = 0; s < b.nsh; s++) {
+        const int l = b.ang_mom[s] - 1, lo = b.sh_loc[s] - 1;
+        const double *r = &b.coords[3 * (size_t)(b.atom_num[s] - 1)];
+        const std::vector<double> &c = l == 0 ? b.cs : (l == 1 ? b.cp : b.cd);
+        shell[s] = make_int4(l, b.contr_num[s], at, 0);
+        xyz[s] = make_double4(r[0], r[1], r[2], 0.0);
+        std::copy(b.exponents.begin() + lo, b.exponents.begin() + lo + b.contr_num[s], ex + at);
+        std::copy(c.begin() + lo, c.begin() + lo + b.contr_num[s], co + at);
+        at += b.contr_num[s];
+    }
+    std::memcpy(host.data() + o_tab, tab.data(), tab.size() * sizeof(double));
+    unsigned char *d = nullptr;
+    CUDA_TRY(cudaMallocAsync((void **)&d, o_out + ntri * sizeof(double), h->stream));
+    h->allocs.push_back(d);
+    CUDA_TRY(cudaMemcpyAsync(d, host.data(), o_out, cudaMemcpyHostToDevice, h->stream));
+    const ShellTable t{(const int4 *)d, (const double4 *)(d + o_xyz), (const double *)(d + o_ex),
+                       (const double *)(d + o_co), (const double *)(d + o_tab), CUX, SQRT_TWOPI52};
+    CUDA_TRY(launch_schwarz_shells(t, b.nsh, (double *)(d + o_out), h->stream));
+    CUDA_TRY(cudaMemcpyAsync(out, d + o_out, ntri * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return LIBERI_OK;
+}
+
 int liberi_c_schwarz(int32_t nsh, int32_t natoms, int32_t num_bas, int32_t mxgtot, const int32_t *ang_mom,
                      const int32_t *contr_num, const int32_t *sh_loc, const int32_t *atom_num,
                      const int32_t *atom_loc, const double *exponents, const double *contr_coef_s,
@@ -2137,10 +2175,16 @@ int liberi_c_schwarz(int32_t nsh, int32_t natoms, int32_t num_bas, int32_t mxgto
     rc = validate_basis(tmp.basis);
     if (rc) return rc;
     CUDA_TRY(cudaGetDevice(&tmp.device));  // the caller's current device
+    CUDA_TRY(high_priority_stream(&tmp.stream));
+    if (std::find(tmp.basis.ang_mom.begin(), tmp.basis.ang_mom.end(), 4) == tmp.basis.ang_mom.end()) {
+        rc = schwarz_shells(&tmp, schwrz_out);
+        free_device(&tmp);
+        return rc;
+    }
+    // f shells: the f classes' evaluation reads pair arrays
     std::vector<double4> shell_xyz;
     build_pairs(tmp.basis, tmp.pairs, shell_xyz);
-    CUDA_TRY(high_priority_stream(&tmp.stream));
-    rc = upload_basis(&tmp, shell_xyz);
+    rc = upload_basis(&tmp, shell_xyz, false);
     double *d_out = nullptr;
     const int npairs = tmp.pairs.class_off[NPC];
     if (!rc) {
@@ -2149,13 +2193,13 @@ int liberi_c_schwarz(int32_t nsh, int32_t natoms, int32_t num_bas, int32_t mxgto
     }
     if (!rc) {
         DevBasis db = dev_basis(&tmp);
-        for (int c = 0; c < NPC && !rc; c++) {
+        // s/p/d pairs in one launch, f ones by the f classes' evaluation
+        cudaError_t e = launch_schwarz(tmp.pairs.class_off, db, tmp.d_tab, d_out, tmp.stream);
+        for (int c = NPC_SPD; c < NPC && e == cudaSuccess; c++) {
             int off = tmp.pairs.class_off[c], n = tmp.pairs.class_off[c + 1] - off;
-            // s/p/d pair classes by their Rys kernels, f ones by the f classes' evaluation
-            cudaError_t e = c < NPC_SPD ? launch_schwarz(c, n, off, db, tmp.d_tab, d_out + off, tmp.stream)
-                                        : launch_fschwarz(c, n, off, db, tmp.d_tab7, d_out, tmp.stream);
-            if (e != cudaSuccess) rc = fail(LIBERI_E_DEVICE, "liberi_schwarz: %s", cudaGetErrorString(e));
+            e = launch_fschwarz(c, n, off, db, tmp.d_tab7, d_out, tmp.stream);
         }
+        if (e != cudaSuccess) rc = fail(LIBERI_E_DEVICE, "liberi_schwarz: %s", cudaGetErrorString(e));
     }
     std::vector<double> per_pair(npairs);
     if (!rc) {

@@ -1,6 +1,6 @@
-// kernels.cu -- class dispatch, Schwarz generator and mixed-precision task
-// builder of the Fock-build engine; the class kernels themselves are
-// instantiated in k_*.cu from quartet.cuh.
+// kernels.cu -- class dispatch and mixed-precision task builder of the
+// Fock-build engine; the class kernels themselves are instantiated in k_*.cu
+// from quartet.cuh.
 #include "unit.cuh"
 
 namespace liberi {
@@ -16,32 +16,6 @@ namespace liberi {
 #define LIBERI_EXTERN(k, a, b, c, d) \
     extern template cudaError_t launch_t<a, b, c, d>(const ClassArgs &, int, int, cudaStream_t);
 LIBERI_CLASSES(LIBERI_EXTERN)
-
-// Schwarz table: sqrt(max |(ab|ab)|) per pair of one class
-template <int LA, int LB>
-__global__ void __launch_bounds__(64) schwarz_kernel(DevBasis b, int pair_off, int npairs,
-                                                     const double *tab, double *out) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npairs) return;
-    const int P = pair_off + t;
-    out[t] = schwarz_diag<LA, LB>(b, P, tab, b.pair_prim0[P], b.pair_nprim[P]);
-}
-
-// Primitive-pair bounds: for every kept primitive pair k of pair P,
-// sqrt(max |(ab|ab)|) of that primitive alone (with its contraction
-// coefficients), rounded up to float: |(ab|cd)_prim| <= out[k] * out[l].
-template <int LA, int LB>
-__global__ void __launch_bounds__(64) prim_bound_kernel(DevBasis b, int pair_off, int npairs, const double *tab,
-                                                        float *out) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npairs) return;
-    const int P = pair_off + t;
-    const int p0 = b.pair_prim0[P], np = b.pair_nprim[P];
-    for (int k = p0; k < p0 + np; k++) {
-        const double v = schwarz_diag<LA, LB>(b, P, tab, k, 1);
-        out[k] = __double2float_ru(v * (1.0 + 1e-6));
-    }
-}
 
 // Per plan item (bra, ket segment, surviving count): split = number of its
 // kets with x_bra*x_ket*max|D| >= fp32_cut (a prefix, the segment is sorted
@@ -100,23 +74,6 @@ __global__ void __launch_bounds__(256) split_tasks_kernel(const __grid_constant_
     const int4 it = s.items[i];
     split_item(it, s.bra_x, s.ket_x, __longlong_as_double((long long)a.maxd[0]), a.fp32_cut, s.chunk ? s.chunk : it.w,
                s.tasks64, s.tasks32, s.counts, 0);
-}
-
-cudaError_t launch_prim_bound(int pc, int npairs, int pair_off, const DevBasis &b, const double *tab, float *out,
-                              cudaStream_t st) {
-    if (npairs <= 0) return cudaSuccess;
-    const int threads = 64;
-    const unsigned blocks = (unsigned)((npairs + threads - 1) / threads);
-    switch (pc) {
-        case SS: prim_bound_kernel<0, 0><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case SP: prim_bound_kernel<1, 0><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case PP: prim_bound_kernel<1, 1><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case SD: prim_bound_kernel<2, 0><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case PD: prim_bound_kernel<2, 1><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case DD: prim_bound_kernel<2, 2><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
 }
 
 // ---- fingerprint of the evaluated quartet set -------------------------------------
@@ -351,23 +308,6 @@ cudaError_t launch_zero_fock(const MolView *d_mols, int nmol, long long max_ntri
     if (blocks > 148 * 16) blocks = 148 * 16;
     if (blocks < 1) blocks = 1;
     zero_fock_kernel<<<(unsigned)blocks, 256, 0, st>>>(d_mols, nmol, max_ntri);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_schwarz(int pc, int npairs, int pair_off, const DevBasis &b, const double *tab, double *out,
-                           cudaStream_t st) {
-    if (npairs <= 0) return cudaSuccess;
-    const int threads = 64;
-    const unsigned blocks = (unsigned)((npairs + threads - 1) / threads);
-    switch (pc) {
-        case SS: schwarz_kernel<0, 0><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case SP: schwarz_kernel<1, 0><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case PP: schwarz_kernel<1, 1><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case SD: schwarz_kernel<2, 0><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case PD: schwarz_kernel<2, 1><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        case DD: schwarz_kernel<2, 2><<<blocks, threads, 0, st>>>(b, pair_off, npairs, tab, out); break;
-        default: return cudaErrorInvalidValue;
-    }
     return cudaGetLastError();
 }
 

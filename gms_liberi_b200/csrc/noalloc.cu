@@ -158,10 +158,7 @@ extern "C" int liberi_c_schwarz_noalloc(int32_t nsh, int32_t natoms, int32_t num
     db.prim_PAf = nullptr;  // the Schwarz kernels are FP64 only
     db.prim_bound = nullptr;
     const double *tab = (const double *)(base + o_tab);
-    for (int c = 0; c < NPC && e == cudaSuccess; c++) {
-        const int o = pairs.class_off[c], n = pairs.class_off[c + 1] - o;
-        e = launch_schwarz(c, n, o, db, tab, d_out + o, 0);
-    }
+    if (e == cudaSuccess) e = launch_schwarz(pairs.class_off, db, tab, d_out, 0);
     std::vector<double> per_pair(npairs);
     if (e == cudaSuccess && npairs > 0)
         e = cudaMemcpy(per_pair.data(), d_out, npairs * sizeof(double), cudaMemcpyDeviceToHost);

@@ -1647,33 +1647,6 @@ __global__ void __launch_bounds__(CLASS_THREADS, PassShape<LA, LB, LC, LD, R, V>
     class_task<LA, LB, LC, LD, R, BATCH, V>(a, a.tasks[blockIdx.x]);
 }
 
-// sqrt(max |(ab|ab)|) over the components of one pair, for the Schwarz table.
-// (primitive pairs p0 .. p0+np-1 of pair P: all of them for the pair's
-// Schwarz value, one for the bound of a single primitive pair)
-template <int LA, int LB>
-__device__ __forceinline__ double schwarz_diag(const DevBasis &b, int P, const double *tab, int p0, int np) {
-    constexpr int NA = ncart(LA), NB = ncart(LB);
-    const int2 sab = b.pair_shell[P];
-    const double4 A = b.shell_xyz[sab.x], B = b.shell_xyz[sab.y];
-    const double abx = A.x - B.x, aby = A.y - B.y, abz = A.z - B.z;
-    double m = 0.0;
-#pragma unroll 1
-    for (int ia = 0; ia < NA; ia++) {
-        double acc[1][NB][NA][NB];
-        eval_block<LA, LB, LA, LB, double, 1, false>(b, p0, np, p0, np, A, A, abx, aby, abz, abx, aby, abz, RYS_TMAX,
-                                              false, tab, nullptr, ia, acc, nullptr, nullptr, 0);
-#pragma unroll
-        for (int ib = 0; ib < NB; ib++) {
-            double v = 0.0;
-#pragma unroll
-            for (int ic = 0; ic < NA; ic++) v = (ic == ia) ? acc[0][ib][ic][ib] : v;
-            v = fabs(v) * s3pow(2 * (cs3_rt(LA, ia) + cs3(LB, ib)));
-            m = v > m ? v : m;
-        }
-    }
-    return sqrt(m);
-}
-
 // A kernel's shared-memory limit and carveout (percent; -1: left alone), set
 // again only when they change: two runtime calls a launch cost as much host
 // time as the launch.  Per device; the values are hints of the launch that
