@@ -36,7 +36,18 @@ __host__ __device__ constexpr int rys_table_off(int n) { return RYS_NINT * RYS_N
 __host__ __device__ constexpr int rys_herm_off(int n) {
     return rys_table_off(MAXROOT + 1) + (n - 1) * 2 * MAXROOT;
 }
-constexpr int RYS_TABLE_SIZE = rys_herm_off(MAXROOT + 1);
+// Boys functions of the Obara-Saika classes (m = 1..4 the highest order), for
+// T <= 25 (their large-T form takes every T above): intervals of width 1/8,
+// per m and interval the degree-7 power-basis coefficients of F_m, then those
+// of exp(-T); the lower orders follow by the downward recursion.
+constexpr int BOYS_MMAX = 4;
+constexpr int BOYS_PER_UNIT = 8;
+constexpr int BOYS_NINT = 25 * BOYS_PER_UNIT + 1;
+constexpr int BOYS_ROW = 2 * RYS_NCOEF;
+__host__ __device__ constexpr int boys_off(int m) {
+    return rys_herm_off(MAXROOT + 1) + (RYS_NCOEF - rys_herm_off(MAXROOT + 1) % RYS_NCOEF) + (m - 1) * BOYS_NINT * BOYS_ROW;
+}
+constexpr int RYS_TABLE_SIZE = boys_off(BOYS_MMAX + 1);
 // Single-precision tables for the FP32 tier: intervals of width 1/8 on
 // [0, RYS_TMAX), degree-3 power basis in x = 2(8T - k) - 1 (4 coefficients:
 // two functions per 256-bit load; interpolation error below 5e-8 relative);
@@ -49,7 +60,14 @@ __host__ __device__ constexpr int rysf_table_off(int n) { return RYSF_NINT * RYS
 __host__ __device__ constexpr int rysf_herm_off(int n) {
     return rysf_table_off(MAXROOT + 1) + (n - 1) * 2 * MAXROOT;
 }
-constexpr int RYSF_TABLE_SIZE = rysf_herm_off(MAXROOT + 1);
+// the Obara-Saika classes' Boys rows in float: degree 3, width 1/8, per m and
+// interval four coefficients of F_m and four of exp(-T) (one 256-bit load)
+constexpr int BOYSF_ROW = 2 * RYSF_NCOEF;
+static_assert(RYSF_PER_UNIT == BOYS_PER_UNIT, "one interval count for both Boys tables");
+__host__ __device__ constexpr int boysf_off(int m) {
+    return rysf_herm_off(MAXROOT + 1) + (8 - rysf_herm_off(MAXROOT + 1) % 8) + (m - 1) * BOYS_NINT * BOYSF_ROW;
+}
+constexpr int RYSF_TABLE_SIZE = boysf_off(BOYS_MMAX + 1);
 // Tables of the f classes: 1..7 roots on [0, RYS7_TMAX) (the 7-root classes
 // switch to the large-T limit at 65), same interval width and degree as above;
 // then per n the large-T limit: MAXROOT7 r_i followed by MAXROOT7 W_i.

@@ -107,15 +107,14 @@ __device__ __forceinline__ void rys_eval(double T, double thr, bool strict,
     }
 }
 
-// Table rows staged in shared memory: the classes with the large-T form from
-// T = 25 (the reference's t_max) need intervals 0..100 only; a CTA copies its
-// class's rows at start, each row padded by 16 bytes (stride 16N+2 doubles)
-// so that lanes reading different rows spread over the banks, and reads them
-// with 128-bit shared loads.  Measured per class on C60 (FP64): (ss|pp)
-// 6.17 -> 5.91 ms, (sp|sp) 14.21 -> 14.11, (ss|dd) 0.353 -> 0.336; slower in
-// the other classes ((ss|ss) 2.78 -> 3.14, (pp|pp) 9.63 -> 10.48, (ss|sd)
-// 1.91 -> 2.22 ms): the copy and the random-row bank conflicts cost more than
-// the L1 misses they save, so only those three stage their rows.
+// Table rows staged in shared memory: a class with the large-T form from
+// T = 25 (the reference's t_max) needs intervals 0..100 only; a CTA copies
+// its class's rows at start, each row padded by 16 bytes (stride 16N+2
+// doubles) so that lanes reading different rows spread over the banks, and
+// reads them with 128-bit shared loads.  Measured on C60 it pays in (ss|dd)
+// alone (0.353 -> 0.336 ms); the copy and the random-row bank conflicts cost
+// the others more than the L1 misses they save ((ss|ss) 2.78 -> 3.14 ms,
+// (pp|pp) 9.63 -> 10.48, and (sp|sp) on Boys rows 11.33 -> 11.50).
 constexpr int STAB_NINT = 25 * RYS_PER_UNIT + 1;
 __host__ __device__ constexpr int stab_stride(int n) { return 16 * n + 2; }
 template <int N>
@@ -150,11 +149,80 @@ __device__ __forceinline__ void rys_eval_staged(double T, double thr, bool stric
         if (f < N) u[f] = v; else w[f - N] = v;
     }
 }
-// the classes that stage their rows (FP64 (ss|pp), (sp|sp), (ss|dd))
+// ---- Boys functions of the Obara-Saika classes ----------------------------------
+// F_0..F_M(T) for the classes with the large-T form above T = 25: one row of
+// F_M and exp(-T) (four 256-bit loads; the two roots and weights of the Rys
+// rule take eight) and the downward recursion, whose terms are all positive.
+template <int M>
+__device__ __forceinline__ void boys_eval(double T, const double *__restrict__ tab, double (&F)[M + 1]) {
+    if (T > 25.0) {
+        const double it = 1.0 / T;
+        F[0] = 0.88622692545275801365 * sqrt(it);
+#pragma unroll
+        for (int m = 1; m <= M; m++) F[m] = F[m - 1] * ((m - 0.5) * it);
+        return;
+    }
+    const double t8 = T * (double)BOYS_PER_UNIT;
+    const int k = (int)t8;
+    const double x = 2.0 * (t8 - (double)k) - 1.0, x2 = x * x, x4 = x2 * x2;
+    double v[2];
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+        double c0, c1, c2, c3, c4, c5, c6, c7;
+        const double *b = tab + boys_off(M) + (size_t)k * BOYS_ROW + f * RYS_NCOEF;
+        ldg_v4f64(b, c0, c1, c2, c3);
+        ldg_v4f64(b + 4, c4, c5, c6, c7);
+        const double a0 = fma(c1, x, c0), a1 = fma(c3, x, c2), a2 = fma(c5, x, c4), a3 = fma(c7, x, c6);
+        v[f] = fma(fma(a3, x2, a2), x4, fma(a1, x2, a0));
+    }
+    F[M] = v[0];
+    const double T2 = 2.0 * T;
+#pragma unroll
+    for (int m = M - 1; m >= 0; m--) F[m] = fma(T2, F[m + 1], v[1]) * (1.0 / (2 * m + 1));
+}
+
+template <int M>
+__device__ __forceinline__ void boys_eval(float T, const float *__restrict__ tabf, float (&F)[M + 1]) {
+    if (T > 25.0f) {
+        const float rs = rsqrtf(T), it = rs * rs;
+        F[0] = 0.886226925f * rs;
+#pragma unroll
+        for (int m = 1; m <= M; m++) F[m] = F[m - 1] * ((m - 0.5f) * it);
+        return;
+    }
+    const float t8 = T * (float)BOYS_PER_UNIT;
+    const int k = (int)t8;
+    const float x = 2.0f * (t8 - (float)k) - 1.0f, x2 = x * x;
+    float4 cf, ce;
+    ldg_v8f32(tabf + boysf_off(M) + (size_t)k * BOYSF_ROW, cf, ce);
+    F[M] = fmaf(fmaf(cf.w, x, cf.z), x2, fmaf(cf.y, x, cf.x));
+    const float e = fmaf(fmaf(ce.w, x, ce.z), x2, fmaf(ce.y, x, ce.x)), T2 = 2.0f * T;
+#pragma unroll
+    for (int m = M - 1; m >= 0; m--) F[m] = fmaf(T2, F[m + 1], e) * (1.0f / (2 * m + 1));
+}
+
+// Classes evaluated by the Obara-Saika recurrences on Boys functions.
+// The single-pass classes with at most one p function beside a shell pair of
+// total angular momentum 1..3.  About half the FP64 operations of the Rys
+// form (one row and the recurrences once a primitive quartet, not once a
+// root) and half its table loads or fewer.  Measured on C60 in FP64:
+// (sp|sp) 13.17 -> 11.33 ms, (sp|pp) 13.28 -> 11.83, (sp|pd) 9.93 -> 8.81,
+// (ss|pp) 6.07 -> 5.09, (sp|sd) 4.30 -> 3.92, (ss|pd) 2.91 -> 2.61,
+// (ss|sd) 1.86 -> 1.62, (ss|sp) 10.89 -> 10.82; the build 103.5 -> 97.2 ms.
+// (On Rys roots as moments the recurrences alone had gained nothing.)
+constexpr bool os_key(int key) {
+    return key == 1000 || key == 1010 || key == 1100 || key == 1110 || key == 2000 || key == 2010 || key == 2100 ||
+           key == 2110;
+}
+template <int LA, int LB, int LC, int LD>
+constexpr bool os_class() {
+    return os_key(LA * 1000 + LB * 100 + LC * 10 + LD);
+}
+// the class that stages its rows (FP64 (ss|dd))
 template <int LA, int LB, int LC, int LD, typename R>
 constexpr bool stab_class() {
     constexpr int key = LA * 1000 + LB * 100 + LC * 10 + LD;
-    return std::is_same<R, double>::value && (key == 1100 || key == 1010 || key == 2200);
+    return std::is_same<R, double>::value && key == 2200;
 }
 template <int LA, int LB, int LC, int LD, typename R>
 constexpr size_t stab_bytes() {
@@ -654,6 +722,64 @@ __device__ __forceinline__ void contract_hgp_pair(const F2 (&gx)[LA + LB + 1][LC
     }
 }
 
+// Obara-Saika contribution of one primitive quartet (S. Obara and A. Saika,
+// J. Chem. Phys. 84 (1986) 3963): c[m] = F_m times the prefactors; pa = P-A,
+// qc = Q-C, wp = W-P, wq = W-Q, hp = 1/2p, rp = q/(p+q), h = 1/2(p+q).
+// add(e, ic, x, y) adds x*y to (e0|c0), e over the functions of angular
+// momentum LA..LA+LB, ic over those of C (LC <= 1).
+__host__ __device__ constexpr int cart_exp(int l, int i, int ax) {
+    return ax == 0 ? cart_x(l, i) : (ax == 1 ? cart_y(l, i) : cart_z(l, i));
+}
+// axis along which component i of l is raised: the one of the smallest nonzero
+// exponent (an exponent of one needs no (a-2) term)
+__host__ __device__ constexpr int raise_axis(int l, int i) {
+    const int x = cart_x(l, i), y = cart_y(l, i), z = cart_z(l, i);
+    return (x > 0 && (y == 0 || x <= y) && (z == 0 || x <= z)) ? 0 : ((y > 0 && (z == 0 || y <= z)) ? 1 : 2);
+}
+// component i of l lowered by k along axis ax (its position within l - k)
+__host__ __device__ constexpr int lower_pos(int l, int i, int ax, int k) {
+    return cart_pos(l - k, cart_x(l, i) - (ax == 0 ? k : 0), cart_y(l, i) - (ax == 1 ? k : 0));
+}
+template <int LA, int LB, int LC, typename R, typename Add>
+__device__ __forceinline__ void os_add(const R (&c)[LA + LB + LC + 1], const R (&pa)[3],
+                                       const R (&qc)[3], const R (&wp)[3], const R (&wq)[3], R hp,
+                                       R rp, R h, Add add) {
+    constexpr int L = LA + LB, M = L + LC;
+    R v[L + 1][M + 1][ncart(L)];  // (a s|s s)^(m), a of angular momentum l: m <= M - l
+#pragma unroll
+    for (int m = 0; m <= M; m++) v[0][m][0] = c[m];
+#pragma unroll
+    for (int l = 1; l <= L; l++)
+#pragma unroll
+        for (int m = 0; m < M; m++)
+#pragma unroll
+            for (int e = 0; e < ncart(L); e++) {
+                if (m > M - l || e >= ncart(l)) continue;
+                const int ax = raise_axis(l, e), n = cart_exp(l, e, ax);
+                const int e1 = lower_pos(l, e, ax, 1);
+                R t = fma(wp[ax], v[l - 1][m + 1][e1], pa[ax] * v[l - 1][m][e1]);
+                if (n > 1) {
+                    const int e2 = lower_pos(l, e, ax, 2), l2 = l > 1 ? l - 2 : 0;
+                    t = fma(R(n - 1) * hp, fma(-rp, v[l2][m + 1][e2], v[l2][m][e2]), t);
+                }
+                v[l][m][e] = t;
+            }
+#pragma unroll
+    for (int e = 0; e < nrange(LA, L); e++) {
+        const int le = range_l(LA, e), ie = range_i(LA, e);
+        if constexpr (LC == 0) add(e, 0, v[le][0][ie], R(1));
+        else {
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                add(e, k, qc[k], v[le][0][ie]);
+                add(e, k, wq[k], v[le][1][ie]);
+                const int n = cart_exp(le, ie, k);
+                if (n > 0) add(e, k, R(n) * h, v[le - 1][1][lower_pos(le, ie, k, 1)]);
+            }
+        }
+    }
+}
+
 // acc[m][ib][ic][id] for A components ia = mu0 + m (m < NMU, ia < NA), all of
 // B, C, D.  A single pass (NMU == NA) uses compile-time component indices; a
 // multi-pass class selects the A exponent at run time, so one copy of the
@@ -706,6 +832,26 @@ __device__ __forceinline__ void eval_block(const DevBasis &b, int p0, int np, in
                 const double2 Px = b.prim_X[kp];
                 const double p = Pp.w, hp = Px.y;
                 const double pqx = Pp.x - Qp.x, pqy = Pp.y - Qp.y, pqz = Pp.z - Qp.z;
+                if constexpr (os_class<LA, LB, LC, LD>() && FULL) {
+                    constexpr int M = LAB + LCD;
+                    const double rs = rsqrt(p + q), ipq = rs * rs;
+                    const double rq = q * ipq, rpp = p * ipq;  // q/(p+q), p/(p+q)
+                    const double T = p * rq * (pqx * pqx + pqy * pqy + pqz * pqz);
+                    double c[M + 1];
+                    boys_eval<M>(T, tab, c);
+                    const double pref = Px.x * Qx.x * rs;
+#pragma unroll
+                    for (int m = 0; m <= M; m++) c[m] *= pref;
+                    const double pa[3] = {Pp.x - A.x, Pp.y - A.y, Pp.z - A.z};
+                    const double qc[3] = {Qp.x - C.x, Qp.y - C.y, Qp.z - C.z};
+                    const double wp[3] = {-rq * pqx, -rq * pqy, -rq * pqz};
+                    const double wq[3] = {rpp * pqx, rpp * pqy, rpp * pqz};
+                    os_add<LA, LB, LC>(c, pa, qc, wp, wq, hp, rq, 0.5 * ipq, [&](int e, int ic, R x, R y) {
+                        if constexpr (HGP) acc[e][ic] = fma(x, y, acc[e][ic]);
+                        else acc[e][0][ic][0] = fma(x, y, acc[e][0][ic][0]);
+                    });
+                    continue;
+                }
                 double u[NR], w[NR];  // u_i / (p+q) and w_i times the pair prefactors
                 if (cache == 2) {
 #pragma unroll
@@ -776,6 +922,24 @@ __device__ __forceinline__ void eval_block(const DevBasis &b, int p0, int np, in
                 ldg_v8f32(PAf + 8 * (size_t)kp, Pp, Pa);
                 const float p = Pp.w, hp = __fdividef(0.5f, p);
                 const float pqx = Pp.x - Qp.x, pqy = Pp.y - Qp.y, pqz = Pp.z - Qp.z;
+                if constexpr (os_class<LA, LB, LC, LD>() && FULL) {
+                    constexpr int M = LAB + LCD;
+                    const float rs = rsqrtf(p + q), ipq = rs * rs;
+                    const float rq = q * ipq, rpp = p * ipq;
+                    const float T = p * q * ipq * (pqx * pqx + pqy * pqy + pqz * pqz);
+                    float c[M + 1];
+                    boys_eval<M>(T, tabf, c);
+                    const float pref = Pa.w * Qa.w * rs;
+#pragma unroll
+                    for (int m = 0; m <= M; m++) c[m] *= pref;
+                    const float pa[3] = {Pa.x, Pa.y, Pa.z}, qc[3] = {Qa.x, Qa.y, Qa.z};
+                    const float wp[3] = {-rq * pqx, -rq * pqy, -rq * pqz}, wq[3] = {rpp * pqx, rpp * pqy, rpp * pqz};
+                    os_add<LA, LB, LC>(c, pa, qc, wp, wq, hp, rq, 0.5f * ipq, [&](int e, int ic, R x, R y) {
+                        if constexpr (HGP) acc[e][ic] = fma(x, y, acc[e][ic]);
+                        else acc[e][0][ic][0] = fma(x, y, acc[e][0][ic][0]);
+                    });
+                    continue;
+                }
                 float u[NR], w[NR];
                 if (cache == 2) {
 #pragma unroll

@@ -168,6 +168,35 @@ std::vector<double> cheb_to_power(const std::vector<double> &f) {
     return pw;
 }
 
+// F_m(T) = exp(-T) sum_k (2T)^k / ((2m+1)(2m+3)...(2m+2k+1)): every term positive
+long double boys_series(int m, long double T) {
+    long double term = 1.0L / (2 * m + 1), sum = term;
+    for (int k = 1; k < 400 && term > 1e-22L * sum; k++) {
+        term *= 2.0L * T / (2 * m + 2 * k + 1);
+        sum += term;
+    }
+    return expl(-T) * sum;
+}
+
+template <typename Real, typename OffT>
+void fill_boys(int M, OffT off, std::vector<Real> &out) {
+    for (int m = 1; m <= BOYS_MMAX; m++)
+        for (int k = 0; k < BOYS_NINT; k++) {
+            std::vector<double> f(M), e(M);
+            for (int i = 0; i < M; i++) {
+                const long double T = (k + 0.5L * (std::cos(PI * (i + 0.5) / M) + 1.0L)) / BOYS_PER_UNIT;
+                f[i] = (double)boys_series(m, T);
+                e[i] = (double)expl(-T);
+            }
+            const std::vector<double> pf = cheb_to_power(f), pe = cheb_to_power(e);
+            Real *dst = &out[off(m) + (size_t)k * 2 * M];
+            for (int i = 0; i < M; i++) {
+                dst[i] = (Real)pf[i];
+                dst[M + i] = (Real)pe[i];
+            }
+        }
+}
+
 // FP32 tier: width-1/8 intervals, degree 3: one float4 per function, the
 // power-basis coefficients small, single-precision evaluation within a few
 // float ulps of the exact roots and weights.
@@ -198,6 +227,7 @@ void build_tables_f32() {
         }
         for (int i = 0; i < 2 * MAXROOT; i++) g_table_f[rysf_herm_off(n) + i] = (float)dt[rys_herm_off(n) + i];
     }
+    fill_boys(RYSF_NCOEF, boysf_off, g_table_f);
 }
 
 // Double-precision table of 1..nmax roots over nint intervals of width
@@ -249,6 +279,7 @@ void fill_table(int nmax, int nint, OffT tab_off, HermT herm_off, std::vector<do
 void build_tables() {
     g_table.assign(RYS_TABLE_SIZE, 0.0);
     fill_table(MAXROOT, RYS_NINT, rys_table_off, rys_herm_off, g_table);
+    fill_boys(RYS_NCOEF, boys_off, g_table);
 }
 
 std::vector<double> g_table7;
