@@ -152,6 +152,12 @@ struct DevPlan {
     const int *ntasks_dev;           // task count on the device (per-build lists) or null
     int ntasks;                      // static count, or capacity for per-build lists
     bool swapped;
+    // merged tasks (first item of a row, first ket and count of the row's
+    // concatenated items, -): the class's items and, for per-build lists, the
+    // FP64 kets of each; null items: tasks name ket positions
+    const int4 *items;
+    const int *split;
+    int threads;             // merged tasks: CTA size
 };
 
 struct RankSplit {
@@ -167,6 +173,10 @@ struct PlanHost {
     int nbra = 0, nket = 0;
     std::vector<int> bra_ids, ket_ids, bra_orig, ket_orig, ncount;
     std::vector<int4> items;  // (bra position, ket segment start, surviving count, -)
+    std::vector<int2> rows;   // per bra position with items: (first item, items)
+    bool merged = false;      // short items: a row's kets run as one range over its items
+    int merged_threads = 128; // CTA size of merged tasks: one warp where rows hold few kets
+    int merged_chunk = 0, merged_cap = 0;  // merged per-build lists: kets per task, capacity
     std::vector<double> bra_x, ket_x;
     std::vector<long long> pref;
     long long total = 0;
@@ -186,6 +196,8 @@ struct PlanHost {
     double *d_bra_x = nullptr, *d_ket_x = nullptr;
     double4 *d_ket_rec = nullptr;
     int4 *d_items = nullptr;
+    int2 *d_rows = nullptr;
+    int *d_split = nullptr;  // mixed: per item its FP64 kets in this build
     int4 *d_tasks = nullptr;
     int4 *d_utasks = nullptr;
     // mixed precision: per-build task lists
@@ -268,15 +280,17 @@ struct LaunchCtx {
 
 cudaError_t launch_class(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs,
                          int precision, int nbf, int tile_rows, int variant);  // precision 0: FP64, 1: FP32
-// f class k (NKERN <= k < NKALL), FP64: one CTA per task, the task's
-// quartets in turn, every quartet evaluated and digested by the whole CTA
+// f class k (NKERN <= k < NKALL), FP64: a group of warps evaluates and digests
+// each quartet of its task
 cudaError_t launch_fclass(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, int nbf);
 // adds {count, sum, xor} of the hashes of the quartets a launch of class k over
 // this plan's task list would evaluate to out[0..2] (zeroed by the caller)
-cudaError_t launch_quartet_fp(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs,
+// (fp32: the list of a mixed build's FP32 kets)
+cudaError_t launch_quartet_fp(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, bool fp32,
                               unsigned long long *out);
-// one launch of class k over the tasks of several molecules (task.w = molecule)
-cudaError_t launch_class_batch(int k, const LaunchCtx &ctx, const int4 *tasks, int ntasks, int nbf_max,
+// one launch of class k over the merged tasks of several molecules (item.w = molecule)
+cudaError_t launch_class_batch(int k, const LaunchCtx &ctx, const int4 *tasks, int ntasks, const int4 *items,
+                               const int *split, int nbf_max,
                                const MolView *d_mols, const ClassView *d_cviews, bool swapped, int precision,
                                const int *ntasks_dev);
 cudaError_t launch_zero_fock(const MolView *d_mols, int nmol, long long max_ntri, cudaStream_t stream);
@@ -284,11 +298,11 @@ cudaError_t launch_zero_fock(const MolView *d_mols, int nmol, long long max_ntri
 // batch its float copy (Df) and max|D| (as ordered bits, maxd non-null)
 cudaError_t launch_batch_prep(const MolView *d_mols, int nmol, long long max_nsq, unsigned long long *maxd,
                               cudaStream_t stream);
-// mixed-precision batch: FP64/FP32 task lists of one class over every molecule's items
-// (item.w = molecule), as split_tasks_kernel does for one molecule
-cudaError_t launch_split_batch(int nitems, const int4 *items, const ClassView *d_cviews,
-                               const unsigned long long *maxd, double fp32_cut, int chunk, int4 *tasks64,
-                               int4 *tasks32, int *counts, cudaStream_t stream);
+// mixed-precision batch: FP64/FP32 task lists of one class over every molecule's
+// rows (first item, items; item.w = molecule)
+cudaError_t launch_split_batch(int nrows, const int2 *rows, const int4 *items, int *split, const ClassView *d_cviews,
+                               const unsigned long long *maxd, double fp32_cut, int4 *tasks64, int4 *tasks32,
+                               int *counts, cudaStream_t stream);
 // start of a build in one launch: F zeroed, the density as a full n x n matrix
 // (and in float where sqf is non-null), the per-build task counters zeroed and,
 // where maxd is non-null (zeroed by the caller), max |D|.  Open-shell builds
@@ -307,11 +321,16 @@ cudaError_t launch_prep(const PrepArgs &a, cudaStream_t st);
 // mixed precision: the FP64 and FP32 task lists of several classes in one launch
 struct SplitClass {
     const int4 *items;
+    const int2 *rows;  // null: one thread an item, kets per task from items[i].w (warp tasks)
+    int *split;
     const double *bra_x, *ket_x;
     int4 *tasks64, *tasks32;
     int *counts;
-    int nitems, chunk, first_block;  // chunk 0: the item's own (items[i].w)
+    int n, first_block;         // rows or items
+    int chunk, merged_chunk;    // kets per task of one item, of a row
+    bool merged32;              // FP32 tasks over the row's concatenated items too (FP64 ones always are)
 };
+constexpr int MERGE_CHUNK = 64;  // kets per merged task of a per-build list where a CTA is one warp
 struct SplitArgs {
     const unsigned long long *maxd;
     double fp32_cut;

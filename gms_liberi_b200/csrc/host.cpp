@@ -214,6 +214,7 @@ struct liberi_handle_s {
     int variant[2][NKERN] = {};  // kernel shape variant per class, FP64 / FP32 tier
     bool timing = false;
     bool last_split_lists = false;  // the last build ran the per-build FP64/FP32 task lists
+    bool last_units = false;        // ... and warp tasks for the classes planned so
     cudaEvent_t ev[NKERN + 1][2] = {};
     bool ev_recorded[NKERN] = {};
     bool plan_dirty = false;
@@ -454,16 +455,89 @@ static double class_max(const PairsHost &pr, int c) {
     return m;
 }
 
-// static CTA tasks of a plan: chunks of at most ph.chunk kets per item; the
-// capacity of the mixed tier's per-build lists follows
-static void build_tasks(PlanHost &ph) {
-    ph.tasks.clear();
-    ph.task_cap = 0;
-    for (const int4 &it : ph.items) {
-        for (int k0 = 0; k0 < it.z; k0 += ph.chunk)
-            ph.tasks.push_back(make_int4(it.x, it.y + k0, std::min(ph.chunk, it.z - k0), 0));
-        ph.task_cap += (it.z + ph.chunk - 1) / ph.chunk + 1;
+// Time in microseconds that one thread spends on a primitive quartet of a class,
+// all passes, in the thread-per-quartet kernels (class times of an ethane-shaped
+// build over its costliest quartet's primitive count): the planner's weights.
+static const double UNIT_US[NKERN] = {0.31, 0.40, 0.62, 0.80, 0.60, 4.0, 0.60, 0.80, 0.80, 1.3, 1.4,
+                                      6.2,  1.4,  1.5,  17.0, 20.0, 6.3, 7.8,  15.0, 60.0, 150.0};
+
+typedef std::vector<std::pair<double, int4>> CostedTasks;  // (estimated time of a lane, task)
+static void by_cost(CostedTasks &lst, std::vector<int4> &out) {
+    std::stable_sort(lst.begin(), lst.end(), [](const std::pair<double, int4> &a, const std::pair<double, int4> &b) {
+        return a.first > b.first;
+    });
+    for (const auto &t : lst) out.push_back(t.second);
+}
+
+// Merged tasks of class k: a row's concatenated items (t.x = item0 + the row's
+// first) cut where a warp has task_us of work (MERGE_TASK_US in one-warp CTAs,
+// so that a task of uncontracted kets pays for its start), at most `cap` kets.
+static const double MERGE_TASK_US = 60.0;
+static void merged_tasks(const PairsHost &pr, const PlanHost &ph, int k, int cap, double task_us, int item0,
+                         CostedTasks &out) {
+    for (const int2 &r : ph.rows) {
+        const double us = UNIT_US[k] * pr.nprim[ph.bra_ids[ph.items[r.x].x]];
+        int f = 0, f0 = 0;     // position in the row, first ket of the open task
+        int next = 0;          // first ket of the next block of 32
+        double cost = 0.0;
+        for (int i = r.x; i < r.x + r.y; i++) {
+            const double block_us = us * pr.kab[ph.ket_ids[ph.items[i].y]];
+            const int end = f + ph.items[i].z;
+            while (next < end) {  // blocks that start in this item
+                if (next > f0 && (cost >= task_us || next - f0 + 32 > cap)) {
+                    out.push_back({cost, make_int4(item0 + r.x, f0, next - f0, 0)});
+                    f0 = next;
+                    cost = 0.0;
+                }
+                cost += block_us;
+                next += 32;
+            }
+            f = end;
+        }
+        if (f > f0) out.push_back({cost, make_int4(item0 + r.x, f0, f - f0, 0)});
     }
+}
+// tasks of at most `chunk` kets of one item each
+static void item_tasks(const PlanHost &ph, int chunk, std::vector<int4> &out) {
+    for (const int4 &it : ph.items)
+        for (int k0 = 0; k0 < it.z; k0 += chunk) out.push_back(make_int4(it.x, it.y + k0, std::min(chunk, it.z - k0), 0));
+}
+static void static_tasks(const PairsHost &pr, int k, PlanHost &ph) {
+    ph.tasks.clear();
+    if (!ph.merged) return item_tasks(ph, ph.chunk, ph.tasks);
+    CostedTasks lst;
+    merged_tasks(pr, ph, k, ph.chunk, ph.merged_threads == 32 ? MERGE_TASK_US : 1e30, 0, lst);
+    by_cost(lst, ph.tasks);
+}
+
+// Rows and static CTA tasks of a plan's items; the capacities of the mixed
+// tier's per-build lists follow.  Rows of fewer than MERGE_ROW_KETS kets run as
+// one-warp CTAs, merged where items average fewer than MERGE_KETS; longer rows
+// keep CLASS_CTA_THREADS and merge items below MERGE_LONG_KETS, but not
+// (ss|ss), whose quartets are too cheap for the walk over items (C60 2.92 ->
+// 3.06 ms).  The FP64 lists of a mixed build are always merged.
+static const double MERGE_ROW_KETS = 700, MERGE_KETS = 400, MERGE_LONG_KETS = 300;
+static void build_tasks(const PairsHost &pr, int k, PlanHost &ph) {
+    ph.rows.clear();
+    ph.task_cap = ph.merged_cap = 0;
+    double kets = 0.0;
+    for (size_t i = 0; i < ph.items.size(); i++) {
+        if (i == 0 || ph.items[i].x != ph.items[i - 1].x) ph.rows.push_back(make_int2((int)i, 0));
+        ph.rows.back().y++;
+        kets += ph.items[i].z;
+        ph.task_cap += (ph.items[i].z + ph.chunk - 1) / ph.chunk + 1;
+    }
+    const bool warp = kets < MERGE_ROW_KETS * ph.rows.size();
+    const double most = warp ? MERGE_KETS : (k == 0 ? 0.0 : MERGE_LONG_KETS);
+    ph.merged = k < NKERN && kets < most * ph.items.size();  // (the f kernels take item tasks)
+    ph.merged_threads = warp ? 32 : CLASS_CTA_THREADS;
+    ph.merged_chunk = warp ? MERGE_CHUNK : ph.chunk;
+    for (const int2 &r : ph.rows) {
+        int n = 0;
+        for (int i = r.x; i < r.x + r.y; i++) n += ph.items[i].z;
+        ph.merged_cap += (n + ph.merged_chunk - 1) / ph.merged_chunk;
+    }
+    static_tasks(pr, k, ph);
 }
 
 static void build_plan(const PairsHost &pr, int k, double cut, int chunk, PlanHost &ph) {
@@ -544,13 +618,13 @@ static void build_plan(const PairsHost &pr, int k, double cut, int chunk, PlanHo
     }
     ph.total = ph.pref[ph.nbra];
     if (ph.chunk <= 0) ph.chunk = default_chunk(k);
-    build_tasks(ph);
+    build_tasks(pr, k, ph);
 }
 
 // Cost-balanced rank split: this rank keeps the contiguous run of items
 // whose cost midpoints fall in its 1/nsize share of the class's primitive-
 // quartet total (cost of an item: nprim(row pair) x sum of its kets' nprim).
-static void balance_items(const PairsHost &pr, int rank, int nsize, PlanHost &ph) {
+static void balance_items(const PairsHost &pr, int k, int rank, int nsize, PlanHost &ph) {
     std::vector<double> cost(ph.items.size());
     double total = 0.0;
     for (size_t i = 0; i < ph.items.size(); i++) {
@@ -568,21 +642,17 @@ static void balance_items(const PairsHost &pr, int rank, int nsize, PlanHost &ph
         before += cost[i];
     }
     ph.items.swap(mine);
-    build_tasks(ph);
+    build_tasks(pr, k, ph);
 }
 
 // Small builds: which classes run as warp tasks (unit.cuh), and how many kets
-// a warp takes of each item.  UNIT_US is the time in microseconds that one
-// thread spends on a primitive quartet of the class, all passes, in the
-// thread-per-quartet kernels (class times of an ethane-shaped build over its
-// costliest quartet's primitive count).  With C the sum of that over the
-// build, an even spread over the GPU's resident lanes takes C / UNIT_LANES; a
-// class goes to warp tasks where its quartets cannot fill the lanes, or where
-// its costliest quartet alone would outlast that even spread.  An item's lanes
-// per quartet are the fewest that bring a quartet below half the even spread,
-// but not below UNIT_FLOOR_US, where a warp's own start and digestion dominate.
-static const double UNIT_US[NKERN] = {0.31, 0.40, 0.62, 0.80, 0.60, 4.0, 0.60, 0.80, 0.80, 1.3, 1.4,
-                                      6.2,  1.4,  1.5,  17.0, 20.0, 6.3, 7.8,  15.0, 60.0, 150.0};
+// a warp takes of each item.  With C the build's UNIT_US over its primitive
+// quartets, an even spread over the GPU's resident lanes takes C / UNIT_LANES;
+// a class goes to warp tasks where its quartets cannot fill the lanes, or
+// where its costliest quartet alone would outlast that even spread.  An item's
+// lanes per quartet are the fewest that bring a quartet below half the even
+// spread, but not below UNIT_FLOOR_US, where a warp's own start and digestion
+// dominate.
 static const double UNIT_LANES = 148 * 16 * 32, UNIT_FLOOR_US = 5.0, UNIT_TAIL_US = 25.0;
 
 static void plan_units(const PairsHost &pr, PlanHost *plans) {
@@ -604,7 +674,7 @@ static void plan_units(const PairsHost &pr, PlanHost *plans) {
         for (const int4 &it : ph.items) q += it.z;
         if ((double)q * UNIT_PG[k] > UNIT_LANES && max_us[k] <= std::max(even_us, UNIT_TAIL_US)) continue;
         ph.unit = true;
-        std::vector<std::pair<double, int4>> lst;
+        CostedTasks lst;
         for (int4 &it : ph.items) {
             const double us = UNIT_US[k] * pr.nprim[ph.bra_ids[it.x]] * pr.kab[ph.ket_ids[it.y]];
             int g = UNIT_PG[k];
@@ -614,10 +684,7 @@ static void plan_units(const PairsHost &pr, PlanHost *plans) {
                 lst.push_back({us / g, make_int4(it.x, it.y + k0, std::min(it.w, it.z - k0), 0)});
             ph.ucap += (it.z + it.w - 1) / it.w + 1;
         }
-        std::stable_sort(lst.begin(), lst.end(), [](const std::pair<double, int4> &a, const std::pair<double, int4> &b) {
-            return a.first > b.first;
-        });
-        for (const auto &t : lst) ph.utasks.push_back(t.second);
+        by_cost(lst, ph.utasks);
     }
 }
 
@@ -634,7 +701,7 @@ static void build_plans(const PairsHost &pr, double cut, const int *chunk, int r
             return;
         }
         build_plan(pr, k, cut, chunk ? chunk[k] : 0, plans[k]);
-        if (rank_split == 1 && nprocs > 1) balance_items(pr, rank, nprocs, plans[k]);
+        if (rank_split == 1 && nprocs > 1) balance_items(pr, k, rank, nprocs, plans[k]);
     };
     std::atomic<int> next{0};
     auto worker = [&]() {
@@ -653,11 +720,6 @@ static void build_plans(const PairsHost &pr, double cut, const int *chunk, int r
     worker();
     for (std::thread &th : pool) th.join();
     plan_units(pr, plans);
-}
-
-static void make_tasks(const PlanHost &ph, int chunk, int mol, std::vector<int4> &out) {
-    for (const int4 &it : ph.items)
-        for (int k0 = 0; k0 < it.z; k0 += chunk) out.push_back(make_int4(it.x, it.y + k0, std::min(chunk, it.z - k0), mol));
 }
 
 // Ket records of a plan (layout beside KET_REC): C - D, C, the first basis
@@ -684,6 +746,9 @@ static void build_ket_records(const BasisHost &b, const PairsHost &pr, const std
 
 static size_t plan_device_bytes(const PlanHost &ph);
 
+// entries of a class's per-build task lists, whichever kind of tasks they hold
+static int list_cap(const PlanHost &ph) { return std::max(ph.task_cap, std::max(ph.ucap, ph.merged_cap)); }
+
 static int upload_plans(liberi_handle h) {
     size_t total = 0;
     for (int k = 0; k < NKALL; k++) total += plan_device_bytes(h->plan[k]);
@@ -704,10 +769,12 @@ static int upload_plans(liberi_handle h) {
         CUDA_TRY(dev_upload(h, &ph.d_bra_x, ph.bra_x.data(), ph.bra_x.size()));
         CUDA_TRY(dev_upload(h, &ph.d_ket_x, ph.ket_x.data(), ph.ket_x.size()));
         CUDA_TRY(dev_upload(h, &ph.d_items, ph.items.data(), ph.items.size()));
+        CUDA_TRY(dev_upload(h, &ph.d_rows, ph.rows.data(), ph.rows.size()));
+        CUDA_TRY(dev_alloc(h, &ph.d_split, ph.items.size()));
         CUDA_TRY(dev_upload(h, &ph.d_tasks, ph.tasks.data(), ph.tasks.size()));
         CUDA_TRY(dev_upload(h, &ph.d_utasks, ph.utasks.data(), ph.utasks.size()));
-        CUDA_TRY(dev_alloc(h, &ph.d_tasks64, (size_t)std::max(ph.task_cap, ph.ucap)));
-        CUDA_TRY(dev_alloc(h, &ph.d_tasks32, (size_t)std::max(ph.task_cap, ph.ucap)));
+        CUDA_TRY(dev_alloc(h, &ph.d_tasks64, (size_t)list_cap(ph)));
+        CUDA_TRY(dev_alloc(h, &ph.d_tasks32, (size_t)list_cap(ph)));
         CUDA_TRY(dev_alloc(h, &ph.d_ntasks, 4));
     }
     return LIBERI_OK;
@@ -720,8 +787,9 @@ static size_t plan_device_bytes(const PlanHost &ph) {
            up_bytes(ph.ket_ids.size(), sizeof(int)) + up_bytes(ph.bra_orig.size(), sizeof(int)) +
            up_bytes(ph.ket_orig.size(), sizeof(int)) + up_bytes(ph.bra_x.size(), sizeof(double)) +
            up_bytes(ph.ket_x.size(), sizeof(double)) + up_bytes(ph.items.size(), sizeof(int4)) +
+           up_bytes(ph.rows.size(), sizeof(int2)) + al_bytes(ph.items.size(), sizeof(int)) +
            up_bytes(ph.tasks.size(), sizeof(int4)) + up_bytes(ph.utasks.size(), sizeof(int4)) +
-           2 * al_bytes((size_t)std::max(ph.task_cap, ph.ucap), sizeof(int4)) +
+           2 * al_bytes((size_t)list_cap(ph), sizeof(int4)) +
            al_bytes(4, sizeof(int));
 }
 
@@ -907,7 +975,7 @@ static int replan(liberi_handle h) {
         // tuner uploaded on its own is released here
         for (void *p : {(void *)ph.d_ket_rec, (void *)ph.d_bra, (void *)ph.d_ket, (void *)ph.d_bra_orig,
                         (void *)ph.d_ket_orig, (void *)ph.d_bra_x, (void *)ph.d_ket_x, (void *)ph.d_items,
-                        (void *)ph.d_tasks, (void *)ph.d_utasks, (void *)ph.d_tasks64, (void *)ph.d_tasks32, (void *)ph.d_ntasks})
+                        (void *)ph.d_rows, (void *)ph.d_split, (void *)ph.d_tasks, (void *)ph.d_utasks, (void *)ph.d_tasks64, (void *)ph.d_tasks32, (void *)ph.d_ntasks})
             if (p) dev_release(h, p);
     }
     if (h->arena_plans.base) dev_release(h, h->arena_plans.base);
@@ -953,6 +1021,9 @@ static DevPlan dev_plan_of(liberi_handle h, int k) {
     dp.ntasks_dev = nullptr;
     dp.ntasks = (int)ph.tasks.size();
     dp.swapped = KDESC[k].swap;
+    dp.items = ph.merged ? ph.d_items : nullptr;
+    dp.split = nullptr;
+    dp.threads = ph.merged_threads;
     return dp;
 }
 
@@ -1006,6 +1077,7 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
     };
     auto runs = [&](int k) { return h->plan[k].total != 0 && ((h->class_mask >> k) & 1u); };
     const bool units = h->units && !h->timing;
+    h->last_units = units;
     {  // F zeroed (liberi_driver.F90:64), D as the class kernels read it
         PrepArgs pa{};
         pa.pa = dD;
@@ -1030,8 +1102,11 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
         for (int k = 0; k < NKERN; k++) {
             const PlanHost &ph = h->plan[k];
             if (!runs(k)) continue;
-            sa.cls[sa.ncls++] = SplitClass{ph.d_items, ph.d_bra_x, ph.d_ket_x, ph.d_tasks64, ph.d_tasks32, ph.d_ntasks,
-                                           (int)ph.items.size(), units && ph.unit ? 0 : ph.chunk, 0};
+            const bool unit = units && ph.unit;
+            sa.cls[sa.ncls++] = SplitClass{ph.d_items, unit ? nullptr : ph.d_rows, ph.d_split, ph.d_bra_x, ph.d_ket_x,
+                                           ph.d_tasks64, ph.d_tasks32, ph.d_ntasks,
+                                           (int)(unit ? ph.items.size() : ph.rows.size()), 0, ph.chunk,
+                                           ph.merged_chunk, ph.merged};
         }
         CUDA_TRY(launch_split_tasks(sa, st));
     }
@@ -1146,12 +1221,16 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
             set_spin(s);
             dp.tasks = mixed ? ph.d_tasks64 : ph.d_tasks;
             dp.ntasks_dev = mixed ? ph.d_ntasks : nullptr;
-            dp.ntasks = mixed ? ph.task_cap : (int)ph.tasks.size();
+            dp.ntasks = mixed ? ph.merged_cap : (int)ph.tasks.size();
+            dp.items = mixed || ph.merged ? ph.d_items : nullptr;
+            dp.split = mixed ? ph.d_split : nullptr;
             ctx.stream = s64;
             CUDA_TRY(launch_class(k, ctx, dp, rs, 0, nbf, tile_rows, h->variant[0][k]));
             if (mixed) {
                 dp.tasks = ph.d_tasks32;
                 dp.ntasks_dev = ph.d_ntasks + 1;
+                dp.ntasks = ph.merged ? ph.merged_cap : ph.task_cap;
+                dp.items = ph.merged ? ph.d_items : nullptr;
                 ctx.stream = s32;
                 CUDA_TRY(launch_class(k, ctx, dp, rs, 1, nbf, tile_rows, h->variant[1][k]));
             }
@@ -1232,11 +1311,13 @@ struct liberi_batch_s {
     int4 *d_tasks[NKERN] = {};
     int ntasks[NKERN] = {};
     int chunk[NKERN] = {};
-    // mixed precision: every molecule's items per class (w = molecule), per-build task lists
+    int4 *d_items[NKERN] = {};  // every molecule's items per class (w = molecule)
+    // mixed precision: their rows, FP64 kets of this iteration and per-build task lists
     int precision = 0;
     double fp32_cut = 0.0, fp32_prim = 0.0;
-    int4 *d_items[NKERN] = {};
-    int nitems[NKERN] = {};
+    int2 *d_rows[NKERN] = {};
+    int *d_split[NKERN] = {};
+    int nrows[NKERN] = {};
     int cap[NKERN] = {};
     int4 *d_t64[NKERN] = {}, *d_t32[NKERN] = {};
     int *d_counts[NKERN] = {};
@@ -1272,7 +1353,13 @@ static void batch_free(liberi_batch b) {
 
 static int batch_build_tasks(liberi_batch b, int k) {
     std::vector<int4> tasks;
-    for (size_t m = 0; m < b->hs.size(); m++) make_tasks(b->hs[m]->plan[k], b->chunk[k], (int)m, tasks);
+    CostedTasks lst;
+    int item0 = 0;
+    for (liberi_handle h : b->hs) {
+        merged_tasks(h->pairs, h->plan[k], k, b->chunk[k], MERGE_TASK_US, item0, lst);
+        item0 += (int)h->plan[k].items.size();
+    }
+    by_cost(lst, tasks);
     if (b->d_tasks[k]) {
         cudaFree(b->d_tasks[k]);
         b->allocs.erase(std::remove(b->allocs.begin(), b->allocs.end(), (void *)b->d_tasks[k]), b->allocs.end());
@@ -1306,18 +1393,25 @@ static int batch_enqueue(liberi_batch b, cudaStream_t st, uint32_t mask) {
     CUDA_TRY(launch_batch_prep(b->d_mols, (int)b->hs.size(), (long long)b->nbf_max * b->nbf_max,
                                mixed ? b->d_maxd : nullptr, st));
     if (!mixed) {
-        for (int k = 0; k < NKERN; k++) {
+        // the classes of few long CTAs at low occupancy run beside the others,
+        // as in large single builds
+        CUDA_TRY(cudaEventRecord(b->fork_ev, st));
+        CUDA_TRY(cudaStreamWaitEvent(b->side, b->fork_ev, 0));
+        for (int k = NKERN - 1; k >= 0; k--) {
             if (!((mask >> k) & 1u) || b->ntasks[k] == 0) continue;
-            CUDA_TRY(launch_class_batch(k, ctx, b->d_tasks[k], b->ntasks[k], b->nbf_max, b->d_mols, b->d_cv[k],
+            ctx.stream = ((h0->side_mask >> k) & 1u) ? b->side : st;
+            CUDA_TRY(launch_class_batch(k, ctx, b->d_tasks[k], b->ntasks[k], b->d_items[k], nullptr, b->nbf_max, b->d_mols, b->d_cv[k],
                                         KDESC[k].swap, 0, nullptr));
         }
+        CUDA_TRY(cudaEventRecord(b->join_ev, b->side));
+        CUDA_TRY(cudaStreamWaitEvent(st, b->join_ev, 0));
         return LIBERI_OK;
     }
     // mixed: every class's task split, then the FP64 lists on the side stream
     // beside the FP32 lists (as for single-molecule builds), joined back
     for (int k = 0; k < NKERN; k++) {
         if (!((mask >> k) & 1u) || b->ntasks[k] == 0) continue;
-        CUDA_TRY(launch_split_batch(b->nitems[k], b->d_items[k], b->d_cv[k], b->d_maxd, b->fp32_cut, b->chunk[k],
+        CUDA_TRY(launch_split_batch(b->nrows[k], b->d_rows[k], b->d_items[k], b->d_split[k], b->d_cv[k], b->d_maxd, b->fp32_cut,
                                     b->d_t64[k], b->d_t32[k], b->d_counts[k], st));
     }
     CUDA_TRY(cudaEventRecord(b->fork_ev, st));
@@ -1325,10 +1419,10 @@ static int batch_enqueue(liberi_batch b, cudaStream_t st, uint32_t mask) {
     for (int k = 0; k < NKERN; k++) {
         if (!((mask >> k) & 1u) || b->ntasks[k] == 0) continue;
         ctx.stream = b->side;
-        CUDA_TRY(launch_class_batch(k, ctx, b->d_t64[k], b->cap[k], b->nbf_max, b->d_mols, b->d_cv[k],
+        CUDA_TRY(launch_class_batch(k, ctx, b->d_t64[k], b->cap[k], b->d_items[k], b->d_split[k], b->nbf_max, b->d_mols, b->d_cv[k],
                                     KDESC[k].swap, 0, b->d_counts[k]));
         ctx.stream = st;
-        CUDA_TRY(launch_class_batch(k, ctx, b->d_t32[k], b->cap[k], b->nbf_max, b->d_mols, b->d_cv[k],
+        CUDA_TRY(launch_class_batch(k, ctx, b->d_t32[k], b->cap[k], b->d_items[k], b->d_split[k], b->nbf_max, b->d_mols, b->d_cv[k],
                                     KDESC[k].swap, 1, b->d_counts[k] + 1));
     }
     CUDA_TRY(cudaEventRecord(b->join_ev, b->side));
@@ -1683,6 +1777,15 @@ int liberi_c_batch_create(liberi_batch *out, const liberi_handle *handles, int32
             return die(fail(LIBERI_E_NOMEM, "liberi_batch_create: out of device memory"));
         b->allocs.push_back(b->d_cv[k]);
         cudaMemcpy(b->d_cv[k], cv.data(), n * sizeof(ClassView), cudaMemcpyHostToDevice);
+        std::vector<int4> items;
+        for (int m = 0; m < n; m++)
+            for (const int4 &it : b->hs[m]->plan[k].items) items.push_back(make_int4(it.x, it.y, it.z, m));
+        if (!items.empty()) {
+            if (cudaMalloc((void **)&b->d_items[k], items.size() * sizeof(int4)) != cudaSuccess)
+                return die(fail(LIBERI_E_NOMEM, "liberi_batch_create: out of device memory"));
+            b->allocs.push_back(b->d_items[k]);
+            cudaMemcpy(b->d_items[k], items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice);
+        }
         b->chunk[k] = default_chunk(k);
         rc = batch_build_tasks(b, k);
         if (rc) return die(rc);
@@ -1707,31 +1810,38 @@ int liberi_c_batch_create(liberi_batch *out, const liberi_handle *handles, int32
         }
     }
     if (b->precision == 1) {
-        // every molecule's items of a class in one list; task capacity for the
-        // smallest kets-per-task the tuner may choose
+        // every molecule's rows of a class in one list
         if (cudaMalloc((void **)&b->d_maxd, n * sizeof(unsigned long long)) != cudaSuccess)
             return die(fail(LIBERI_E_NOMEM, "liberi_batch_create: out of device memory"));
         b->allocs.push_back(b->d_maxd);
         for (int k = 0; k < NKERN; k++) {
-            std::vector<int4> items;
+            std::vector<int2> rows;
             long long cap = 0;
-            for (int m = 0; m < n; m++)
-                for (const int4 &it : b->hs[m]->plan[k].items) {
-                    items.push_back(make_int4(it.x, it.y, it.z, m));
-                    cap += (it.z + TUNE_CHUNKS[0] - 1) / TUNE_CHUNKS[0] + 1;
+            int item0 = 0;
+            for (int m = 0; m < n; m++) {
+                const PlanHost &ph = b->hs[m]->plan[k];
+                for (const int2 &r : ph.rows) {
+                    rows.push_back(make_int2(item0 + r.x, r.y));
+                    int nk = 0;
+                    for (int i = r.x; i < r.x + r.y; i++) nk += ph.items[i].z;
+                    cap += (nk + MERGE_CHUNK - 1) / MERGE_CHUNK;
                 }
-            if (items.empty()) continue;
+                item0 += (int)ph.items.size();
+            }
+            if (rows.empty()) continue;
             if (cap > INT32_MAX) return die(fail(LIBERI_E_UNSUPPORTED, "liberi_batch_create: batch too large"));
-            b->nitems[k] = (int)items.size();
+            b->nrows[k] = (int)rows.size();
             b->cap[k] = (int)cap;
-            if (cudaMalloc((void **)&b->d_items[k], items.size() * sizeof(int4)) != cudaSuccess ||
+            if (cudaMalloc((void **)&b->d_rows[k], rows.size() * sizeof(int2)) != cudaSuccess ||
+                cudaMalloc((void **)&b->d_split[k], (size_t)item0 * sizeof(int)) != cudaSuccess ||
                 cudaMalloc((void **)&b->d_t64[k], cap * sizeof(int4)) != cudaSuccess ||
                 cudaMalloc((void **)&b->d_t32[k], cap * sizeof(int4)) != cudaSuccess ||
                 cudaMalloc((void **)&b->d_counts[k], 4 * sizeof(int)) != cudaSuccess)
                 return die(fail(LIBERI_E_NOMEM, "liberi_batch_create: out of device memory"));
-            for (void *p : {(void *)b->d_items[k], (void *)b->d_t64[k], (void *)b->d_t32[k], (void *)b->d_counts[k]})
+            for (void *p : {(void *)b->d_rows[k], (void *)b->d_split[k], (void *)b->d_t64[k], (void *)b->d_t32[k],
+                            (void *)b->d_counts[k]})
                 b->allocs.push_back(p);
-            cudaMemcpy(b->d_items[k], items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice);
+            cudaMemcpy(b->d_rows[k], rows.data(), rows.size() * sizeof(int2), cudaMemcpyHostToDevice);
         }
     }
     *out = b;
@@ -1901,8 +2011,7 @@ int liberi_c_autotune(liberi_handle h, int32_t reps, int32_t *chunks_out) {
             for (int c : TUNE_CHUNKS) {
                 PlanHost &ph = h->plan[k];
                 ph.chunk = c;
-                ph.tasks.clear();
-                make_tasks(ph, c, 0, ph.tasks);
+                static_tasks(h->pairs, k, ph);
                 if (ph.d_tasks) {  // used only by this tuner's builds on the handle's stream
                     dev_release(h, ph.d_tasks);
                     ph.d_tasks = nullptr;
@@ -2095,18 +2204,22 @@ static int quartet_fingerprint(liberi_handle h, int nclass, uint64_t *out) {
         const RankSplit rs = rank_split_of(h, k);
         DevPlan dp = dev_plan_of(h, k);
         if (!h->last_split_lists || k >= NKERN) {  // f classes: always the static FP64 list
-            e = launch_quartet_fp(k, ctx, dp, rs, d_out + 3 * k);
+            e = launch_quartet_fp(k, ctx, dp, rs, false, d_out + 3 * k);
             continue;
         }
         // the lists the last (mixed-precision) build split and launched
-        dp.ntasks = std::max(ph.task_cap, ph.ucap);
+        const bool unit = h->last_units && ph.unit;
+        dp.ntasks = list_cap(ph);
         dp.tasks = ph.d_tasks64;
         dp.ntasks_dev = ph.d_ntasks;
-        e = launch_quartet_fp(k, ctx, dp, rs, d_out + 3 * k);
+        dp.items = unit ? nullptr : ph.d_items;
+        dp.split = ph.d_split;
+        e = launch_quartet_fp(k, ctx, dp, rs, false, d_out + 3 * k);
         if (e != cudaSuccess) break;
         dp.tasks = ph.d_tasks32;
         dp.ntasks_dev = ph.d_ntasks + 1;
-        e = launch_quartet_fp(k, ctx, dp, rs, d_out + 3 * k);
+        dp.items = !unit && ph.merged ? ph.d_items : nullptr;
+        e = launch_quartet_fp(k, ctx, dp, rs, true, d_out + 3 * k);
     }
     unsigned long long host[3 * NKALL];
     if (e == cudaSuccess) e = cudaMemcpyAsync(host, d_out, sizeof(host), cudaMemcpyDeviceToHost, st);

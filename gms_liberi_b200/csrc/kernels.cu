@@ -33,35 +33,43 @@ __device__ __forceinline__ int item_split(const int4 &it, const double *bra_x, c
     return lo;
 }
 
-// One thread per item: the split point, then output ranges reserved with
-// atomics (task order only affects load balance).  counts[0..1]: FP64 and
-// FP32 task counts, counts[2..3]: FP32 quartet count (64-bit, low word first);
-// zeroed before the launch.
-__device__ __forceinline__ void split_item(const int4 &it, const double *bx, const double *kx, double maxd,
-                                           double fp32_cut, int chunk, int4 *tasks64, int4 *tasks32, int *counts,
-                                           int w) {
-    const int s = item_split(it, bx, kx, maxd, fp32_cut);
-    const int n64 = (s + chunk - 1) / chunk, n32 = (it.z - s + chunk - 1) / chunk;
-    if (n64) {
-        int o = atomicAdd(counts, n64);
-        for (int k = 0; k < s; k += chunk) tasks64[o++] = make_int4(it.x, it.y + k, min(chunk, s - k), w);
-    }
-    if (n32) {
-        int o = atomicAdd(counts + 1, n32);
-        for (int k = s; k < it.z; k += chunk) tasks32[o++] = make_int4(it.x, it.y + k, min(chunk, it.z - k), w);
-        atomicAdd(reinterpret_cast<unsigned long long *>(counts + 2), (unsigned long long)(it.z - s));
-    }
+// Output ranges are reserved with atomics (task order only affects load
+// balance).  counts[0..1]: FP64 and FP32 task counts, counts[2..3]: FP32
+// quartet count (64-bit, low word first); zeroed before the launch.
+__device__ __forceinline__ void emit_tasks(int x, int y, int n, int chunk, int4 *tasks, int *count) {
+    if (n <= 0) return;
+    int o = atomicAdd(count, (n + chunk - 1) / chunk);
+    for (int k = 0; k < n; k += chunk) tasks[o++] = make_int4(x, y + k, min(chunk, n - k), 0);
 }
-// batch: item.w is the molecule, whose Schwarz lists and max|D| are used and
-// which the tasks carry
-__global__ void __launch_bounds__(256) split_batch_kernel(int nitems, const int4 *items, const ClassView *cviews,
+// One row: its items' split points, and merged tasks over the FP64 kets of
+// all its items (a row holds few of them per contraction pattern: a C60 build
+// at cut 1e-5 some tens); the FP32 kets item by item or merged.
+__device__ __forceinline__ void split_row(int2 row, const int4 *items, int *split, const double *bx, const double *kx,
+                                          double maxd, double fp32_cut, int chunk, int mchunk, bool merged32,
+                                          int4 *tasks64, int4 *tasks32, int *counts) {
+    int c64 = 0, c32 = 0;
+    for (int i = row.x; i < row.x + row.y; i++) {
+        const int4 it = items[i];
+        const int s = item_split(it, bx, kx, maxd, fp32_cut);
+        split[i] = s;
+        c64 += s;
+        c32 += it.z - s;
+        if (!merged32) emit_tasks(it.x, it.y + s, it.z - s, chunk, tasks32, counts + 1);
+    }
+    emit_tasks(row.x, 0, c64, mchunk, tasks64, counts);
+    if (merged32) emit_tasks(row.x, 0, c32, mchunk, tasks32, counts + 1);
+    if (c32) atomicAdd(reinterpret_cast<unsigned long long *>(counts + 2), (unsigned long long)c32);
+}
+// batch: item.w is the molecule, whose Schwarz lists and max|D| are used
+__global__ void __launch_bounds__(256) split_batch_kernel(int nrows, const int2 *rows, const int4 *items, int *split,
+                                                          const ClassView *cviews,
                                                           const unsigned long long *maxd_bits, double fp32_cut,
-                                                          int chunk, int4 *tasks64, int4 *tasks32, int *counts) {
+                                                          int4 *tasks64, int4 *tasks32, int *counts) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    const int4 it = items[i];
-    split_item(it, cviews[it.w].bra_x, cviews[it.w].ket_x, __longlong_as_double((long long)maxd_bits[it.w]), fp32_cut,
-               chunk, tasks64, tasks32, counts, it.w);
+    if (i >= nrows) return;
+    const int w = items[rows[i].x].w;
+    split_row(rows[i], items, split, cviews[w].bra_x, cviews[w].ket_x, __longlong_as_double((long long)maxd_bits[w]),
+              fp32_cut, 0, MERGE_CHUNK, true, tasks64, tasks32, counts);
 }
 // one molecule: every class of the build in one launch (21 launches and 21
 // counter resets cost a 10-atom mixed build about 100 us of host time)
@@ -70,10 +78,18 @@ __global__ void __launch_bounds__(256) split_tasks_kernel(const __grid_constant_
     while (c + 1 < a.ncls && (int)blockIdx.x >= a.cls[c + 1].first_block) c++;
     const SplitClass &s = a.cls[c];
     const int i = ((int)blockIdx.x - s.first_block) * blockDim.x + threadIdx.x;
-    if (i >= s.nitems) return;
+    if (i >= s.n) return;
+    const double maxd = __longlong_as_double((long long)a.maxd[0]);
+    if (s.rows) {
+        split_row(s.rows[i], s.items, s.split, s.bra_x, s.ket_x, maxd, a.fp32_cut, s.chunk, s.merged_chunk,
+                  s.merged32, s.tasks64, s.tasks32, s.counts);
+        return;
+    }
     const int4 it = s.items[i];
-    split_item(it, s.bra_x, s.ket_x, __longlong_as_double((long long)a.maxd[0]), a.fp32_cut, s.chunk ? s.chunk : it.w,
-               s.tasks64, s.tasks32, s.counts, 0);
+    const int n64 = item_split(it, s.bra_x, s.ket_x, maxd, a.fp32_cut);
+    emit_tasks(it.x, it.y, n64, it.w, s.tasks64, s.counts);
+    emit_tasks(it.x, it.y + n64, it.z - n64, it.w, s.tasks32, s.counts + 1);
+    if (it.z > n64) atomicAdd(reinterpret_cast<unsigned long long *>(s.counts + 2), (unsigned long long)(it.z - n64));
 }
 
 // ---- fingerprint of the evaluated quartet set -------------------------------------
@@ -98,15 +114,19 @@ __device__ __forceinline__ unsigned long long quartet_fp(int2 ab, int2 cd) {
     return fp_mix64(p1 > p2 ? (p1 << 32 | p2) : (p2 << 32 | p1));
 }
 
-__global__ void __launch_bounds__(CLASS_THREADS) quartet_fp_kernel(ClassArgs a, unsigned long long *out) {
+__global__ void __launch_bounds__(CLASS_THREADS) quartet_fp_kernel(ClassArgs a, bool fp32, unsigned long long *out) {
     const int ntasks = a.ntasks_dev ? *a.ntasks_dev : a.ntasks;
     if ((int)blockIdx.x >= ntasks) return;
     const int4 t = a.tasks[blockIdx.x];
-    const int2 ab = a.b.pair_shell[a.bra_ids[t.x]];
+    const int ibra = a.items ? a.items[t.x].x : t.x;
+    const int2 ab = a.b.pair_shell[a.bra_ids[ibra]];
     unsigned long long n = 0, sum = 0, x = 0;
     for (int qi = threadIdx.x; qi < t.z; qi += CLASS_THREADS) {
-        const int j = t.y + qi;
-        if (!quartet_owned(a, t.x, j)) continue;
+        int j = t.y + qi;
+        if (a.items)
+            j = fp32 ? merged_ket<float>(a.items + t.x, a.split + t.x, j)
+                     : merged_ket<double>(a.items + t.x, a.split ? a.split + t.x : nullptr, j);
+        if (!quartet_owned(a, ibra, j)) continue;
         const unsigned long long f = quartet_fp(ab, a.b.pair_shell[a.ket_ids[j]]);
         n++;
         sum += f;
@@ -128,11 +148,11 @@ __global__ void __launch_bounds__(CLASS_THREADS) quartet_fp_kernel(ClassArgs a, 
 static ClassArgs single_args(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, int nbf,
                              int tile_rows);
 
-cudaError_t launch_quartet_fp(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs,
+cudaError_t launch_quartet_fp(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, bool fp32,
                               unsigned long long *out) {
     if (plan.ntasks <= 0) return cudaSuccess;
     const ClassArgs a = single_args(k, ctx, plan, rs, 0, 0);
-    quartet_fp_kernel<<<(unsigned)plan.ntasks, CLASS_THREADS, 0, ctx.stream>>>(a, out);
+    quartet_fp_kernel<<<(unsigned)plan.ntasks, CLASS_THREADS, 0, ctx.stream>>>(a, fp32, out);
     return cudaGetLastError();
 }
 
@@ -170,6 +190,9 @@ static ClassArgs single_args(int k, const LaunchCtx &ctx, const DevPlan &plan, c
     a.ket_rec = plan.ket_rec;
     a.bra_orig = plan.bra_orig;
     a.ket_orig = plan.ket_orig;
+    a.items = plan.items;
+    a.split = plan.split;
+    a.threads = plan.threads;
     a.swapped = plan.swapped ? 1 : 0;
     a.rs = rs;
     a.mols = nullptr;
@@ -180,7 +203,8 @@ static ClassArgs single_args(int k, const LaunchCtx &ctx, const DevPlan &plan, c
     return a;
 }
 
-cudaError_t launch_class_batch(int k, const LaunchCtx &ctx, const int4 *tasks, int ntasks, int nbf_max,
+cudaError_t launch_class_batch(int k, const LaunchCtx &ctx, const int4 *tasks, int ntasks, const int4 *items,
+                               const int *split, int nbf_max,
                                const MolView *d_mols, const ClassView *d_cviews, bool swapped, int precision,
                                const int *ntasks_dev) {
     const KernelDesc &kd = KDESC[k];
@@ -203,6 +227,9 @@ cudaError_t launch_class_batch(int k, const LaunchCtx &ctx, const int4 *tasks, i
     a.tile_rows = 0;
     a.bra_ids = a.ket_ids = a.bra_orig = a.ket_orig = nullptr;
     a.ket_rec = nullptr;
+    a.items = items;
+    a.split = split;
+    a.threads = 32;
     a.swapped = swapped ? 1 : 0;
     a.rs = RankSplit{0, 1, 0, 0, 0, 0, 0, 0};
     a.mols = d_mols;
@@ -315,7 +342,7 @@ cudaError_t launch_split_tasks(SplitArgs a, cudaStream_t st) {
     int blocks = 0;
     for (int c = 0; c < a.ncls; c++) {
         a.cls[c].first_block = blocks;
-        blocks += (a.cls[c].nitems + 255) / 256;
+        blocks += (a.cls[c].n + 255) / 256;
     }
     if (blocks == 0) return cudaSuccess;
     split_tasks_kernel<<<(unsigned)blocks, 256, 0, st>>>(a);
@@ -371,13 +398,13 @@ cudaError_t launch_units(bool low, int ncls, const int *ks, const LaunchCtx &ctx
                           : launch_unit_t<false, float>(a, blocks, ctx.stream);
 }
 
-cudaError_t launch_split_batch(int nitems, const int4 *items, const ClassView *d_cviews,
-                               const unsigned long long *maxd, double fp32_cut, int chunk, int4 *tasks64,
-                               int4 *tasks32, int *counts, cudaStream_t st) {
+cudaError_t launch_split_batch(int nrows, const int2 *rows, const int4 *items, int *split, const ClassView *d_cviews,
+                               const unsigned long long *maxd, double fp32_cut, int4 *tasks64, int4 *tasks32,
+                               int *counts, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(counts, 0, 4 * sizeof(int), st);
-    if (e != cudaSuccess || nitems <= 0) return e;
-    split_batch_kernel<<<(nitems + 255) / 256, 256, 0, st>>>(nitems, items, d_cviews, maxd, fp32_cut, chunk, tasks64,
-                                                             tasks32, counts);
+    if (e != cudaSuccess || nrows <= 0) return e;
+    split_batch_kernel<<<(nrows + 255) / 256, 256, 0, st>>>(nrows, rows, items, split, d_cviews, maxd, fp32_cut, tasks64,
+                                                            tasks32, counts);
     return cudaGetLastError();
 }
 

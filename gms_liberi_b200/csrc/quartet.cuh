@@ -1317,14 +1317,14 @@ constexpr bool root_cache_on(int key, bool f32) { return !f32 && key != 2121; }
 // Per-quartet partial sums that outlive a pass: K updates of the B rows
 // (bc[ib][ic], bd[ib][id]) and the ket-pair J block (cd[ic][id]).  Single-
 // pass classes keep them in registers; multi-pass classes in per-thread
-// shared-memory slots (stride CLASS_THREADS, bank-conflict free).
-template <int NB, int NC, int ND, bool SM, typename T>
+// shared-memory slots (stride the CTA size, bank-conflict free).
+template <int NB, int NC, int ND, bool SM, bool MERGED, typename T>
 struct KBuf {
     static constexpr int N = NB * NC + NB * ND + NC * ND;
     T r[SM ? 1 : N];
     T *s;
     __device__ __forceinline__ T &at(int i) {
-        if constexpr (SM) return s[i * CLASS_THREADS];
+        if constexpr (SM) return s[i * (MERGED ? (int)blockDim.x : CLASS_THREADS)];
         else return r[i];
     }
     __device__ __forceinline__ T &bc(int ib, int ic) { return at(ib * NC + ic); }
@@ -1613,7 +1613,10 @@ struct ClassArgs {
     double cut;
     double thr;
     bool strict;
-    const int4 *tasks;       // (bra position, first ket position, ket count, -)
+    const int4 *tasks;       // (bra position, first ket position, ket count, -), or merged (engine.h DevPlan)
+    const int4 *items;       // merged tasks: the class's items, and their FP64 kets in this build
+    const int *split;
+    int threads;             // merged tasks: CTA size, 32 or CLASS_THREADS
     const int *ntasks_dev;   // device task count (per-build task lists) or null
     int ntasks;              // static task count / grid bound
     int nbf;
@@ -1674,14 +1677,39 @@ __device__ __forceinline__ const double4 *mol_ketrec(const ClassArgs &a, int w) 
     if constexpr (BATCH) return a.cviews[w].ket_rec; else return a.ket_rec;
 }
 
+// Merged tasks: ket position of the f-th ket of a row, its items (from the
+// row's first) one after another; with split counts the FP64 kets are the
+// first split[i] of item i and the FP32 kets the rest.  f is below the row's
+// total, so the walk ends inside the row.
+template <typename R>
+__device__ __forceinline__ int merged_ket(const int4 *__restrict__ items, const int *__restrict__ split, int f) {
+    for (int i = 0;; i++) {
+        const int4 it = items[i];
+        const int s = split ? split[i] : it.z;
+        const int n = std::is_same<R, float>::value ? it.z - s : s;
+        if (f < n) return it.y + f + (std::is_same<R, float>::value ? s : 0);
+        f -= n;
+    }
+}
+
 // One CTA task: row pair t.x against kets t.y .. t.y+t.z-1 of one molecule.
-template <int LA, int LB, int LC, int LD, typename R, bool BATCH, int V>
-__device__ __forceinline__ void class_task(const ClassArgs &a, const int4 t) {
+// MERGED: a range over the concatenated items of the row whose first item is
+// t.x.  A row of a small molecule, or the FP64 kets of a row in a mixed build,
+// are 10 to 60 kets of one contraction pattern, so that tasks of one pattern
+// each leave lanes of most warps idle.  Rows of few kets run one warp per CTA:
+// a row's kets are ordered by contraction, so the warps of a larger CTA would
+// hold quartets of 81, 27, 9 ... primitives and its registers would wait for
+// the first (a batch of 40 molecules: 62.5 ms on item tasks with its classes
+// in turn, 52.0 merged with 128 threads, 44.3 with 32); rows of many kets keep
+// 128 threads, whose warps share the row's data in L1 (mixed C60 at cut 1e-5,
+// FP64 lists: 62.3 ms against 65.7 with 32).
+template <int LA, int LB, int LC, int LD, typename R, bool BATCH, bool MERGED, int V>
+__device__ __forceinline__ void class_task(const ClassArgs &a, int4 t) {
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     extern __shared__ __align__(16) unsigned char class_smem[];
     // the class's staged table rows come first (16-byte aligned), then the
-    // F-row tile and the per-thread slots (batched launches do not stage)
-    constexpr size_t STB = BATCH ? 0 : stab_bytes<LA, LB, LC, LD, R>();
+    // F-row tile and the per-thread slots (merged tasks do neither stage nor tile)
+    constexpr size_t STB = MERGED ? 0 : stab_bytes<LA, LB, LC, LD, R>();
     const double *stab = nullptr;
     if constexpr (STB > 0) {
         constexpr int NRt = (LA + LB + LC + LD) / 2 + 1;
@@ -1696,6 +1724,14 @@ __device__ __forceinline__ void class_task(const ClassArgs &a, const int4 t) {
         if (a.thr <= 25.0) stab = st;
     }
     R *tile = reinterpret_cast<R *>(class_smem + STB);  // the digestion type: FP32 tile for the FP32 tier
+    const int4 *items = nullptr;
+    const int *split = nullptr;
+    if constexpr (MERGED) {
+        items = a.items + t.x;
+        split = a.split ? a.split + t.x : nullptr;
+        t.x = items[0].x;
+        t.w = items[0].w;
+    }
     const int ibra = t.x, k0 = t.y, cnt = t.z;
     const DevBasis &bas = mol_basis<BATCH>(a, t.w);
 #define LIBERI_D mol_D<BATCH, R>(a, t.w)
@@ -1710,7 +1746,7 @@ __device__ __forceinline__ void class_task(const ClassArgs &a, const int4 t) {
     // accesses) only when the task's kets touch a fair part of each row;
     // short tasks (the FP64 head of a mixed-precision item, item tails) add
     // their K updates to F directly
-    const bool use_tile = a.tile_rows != 0 && 4 * cnt * (NC + ND) >= LIBERI_NBF;
+    const bool use_tile = !MERGED && a.tile_rows != 0 && 4 * cnt * (NC + ND) >= LIBERI_NBF;
     if (use_tile) {
         for (int i = threadIdx.x; i < nrow * LIBERI_NBF; i += CLASS_THREADS) tile[i] = R(0);
         __syncthreads();
@@ -1739,10 +1775,11 @@ __device__ __forceinline__ void class_task(const ClassArgs &a, const int4 t) {
     // quartets per trip, lanes 0..G-1 the first, and so on.
     constexpr int G = PassShape<LA, LB, LC, LD, R, V>::TPQ;
     const int gsub = (int)(threadIdx.x & 31) & (G - 1);
-    for (int qb = (int)(threadIdx.x >> 5) * (32 / G); qb < cnt; qb += CLASS_THREADS / G) {
+    for (int qb = (int)(threadIdx.x >> 5) * (32 / G); qb < cnt; qb += (MERGED ? (int)blockDim.x : CLASS_THREADS) / G) {
         const int qi = qb + (int)(threadIdx.x & 31) / G;
         bool act = qi < cnt;
-        const int j = k0 + (act ? qi : 0);
+        int j = k0 + (act ? qi : 0);
+        if constexpr (MERGED) j = merged_ket<R>(items, split, j);
         if (act && a.rs.nsize > 1) act = quartet_owned(a, ibra, j);
         const double4 *krec = mol_ketrec<BATCH>(a, t.w) + KET_REC * j;
         const double4 r0 = ldg_double4(krec), r1 = ldg_double4(krec + 1);
@@ -1758,17 +1795,17 @@ __device__ __forceinline__ void class_task(const ClassArgs &a, const int4 t) {
         qc.cut = R(a.cut); qc.Dm = LIBERI_D; qc.ld = (unsigned)LIBERI_NBF;
         qc.DmK = LIBERI_D + a.k_offset;  // open-shell builds: the exchange density follows D
         constexpr bool SM = PassShape<LA, LB, LC, LD, R, V>::NPASS > 1;
-        KBuf<NB, NC, ND, SM, R> kb;
+        KBuf<NB, NC, ND, SM, MERGED, R> kb;
         kb.s = slots + threadIdx.x;
 #pragma unroll
-        for (int i = 0; i < KBuf<NB, NC, ND, SM, R>::N; i++) kb.at(i) = R(0);
+        for (int i = 0; i < KBuf<NB, NC, ND, SM, MERGED, R>::N; i++) kb.at(i) = R(0);
         run_passes<LA, LB, LC, LD, R, V>(bas, p0, np, (int)(unsigned)kpr, act ? (int)(unsigned)(kpr >> 32) : 0, A, C, abx, aby,
                                       abz, cdx, cdy, cdz, a.thr, a.strict, a.tab, a.tabf, qc, rowsA, kb, pthr, bpmax, stab);
         if constexpr (G > 1) {
             // the group's lanes hold partial sums over their passes: combine
             // them, the group's first lane adds them to F
 #pragma unroll
-            for (int i = 0; i < KBuf<NB, NC, ND, SM, R>::N; i++) kb.at(i) = group_sum<G>(kb.at(i));
+            for (int i = 0; i < KBuf<NB, NC, ND, SM, MERGED, R>::N; i++) kb.at(i) = group_sum<G>(kb.at(i));
         }
         if (G == 1 || gsub == 0) {
 #pragma unroll
@@ -1802,13 +1839,13 @@ __device__ __forceinline__ void class_task(const ClassArgs &a, const int4 t) {
 #undef LIBERI_NBF
 }
 
-// BATCH: the task's w field selects the molecule (basis, D, F, plan lists);
-// the launch sized the shared-memory tile for the largest molecule.
-template <int LA, int LB, int LC, int LD, typename R, bool BATCH, int V>
+// BATCH (always merged): the item's w field selects the molecule (basis, D, F,
+// plan lists).
+template <int LA, int LB, int LC, int LD, typename R, bool BATCH, bool MERGED, int V>
 __global__ void __launch_bounds__(CLASS_THREADS, PassShape<LA, LB, LC, LD, R, V>::MINB) class_kernel(ClassArgs a) {
     const int ntasks = a.ntasks_dev ? *a.ntasks_dev : a.ntasks;
     if ((int)blockIdx.x >= ntasks) return;  // lists counted on the device launch their capacity
-    class_task<LA, LB, LC, LD, R, BATCH, V>(a, a.tasks[blockIdx.x]);
+    class_task<LA, LB, LC, LD, R, BATCH, MERGED, V>(a, a.tasks[blockIdx.x]);
 }
 
 // A kernel's shared-memory limit and carveout (percent; -1: left alone), set
@@ -1831,11 +1868,12 @@ struct FuncAttrs {
     }
 };
 
-template <int LA, int LB, int LC, int LD, typename R, bool BATCH, int V>
+template <int LA, int LB, int LC, int LD, typename R, bool BATCH, bool MERGED, int V>
 cudaError_t launch_shape(const ClassArgs &a, cudaStream_t st) {
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     constexpr bool SM = PassShape<LA, LB, LC, LD, R, V>::NPASS > 1;
-    const size_t slot_bytes = SM ? (size_t)KBuf<NB, NC, ND, true, R>::N * CLASS_THREADS * sizeof(R) : 0;
+    const int threads = MERGED ? a.threads : CLASS_THREADS;
+    const size_t slot_bytes = SM ? (size_t)KBuf<NB, NC, ND, true, MERGED, R>::N * threads * sizeof(R) : 0;
     // the F-row tile is staged only when it fits beside the slots (227 KB per CTA)
     const size_t tile_bytes = (size_t)(NA + NB) * a.nbf * sizeof(R);
     // The F-row tile is staged only when it fits beside the slots at the
@@ -1844,8 +1882,8 @@ cudaError_t launch_shape(const ClassArgs &a, cudaStream_t st) {
     // the global atomics it saves.
     constexpr int MINB = PassShape<LA, LB, LC, LD, R, V>::MINB;
     ClassArgs args = a;
-    constexpr size_t STB = BATCH ? 0 : stab_bytes<LA, LB, LC, LD, R>();
-    args.tile_rows = (a.tile_rows && (tile_bytes + slot_bytes + STB) * MINB <= CLASS_DYN_SMEM_MAX) ? 1 : 0;
+    constexpr size_t STB = MERGED ? 0 : stab_bytes<LA, LB, LC, LD, R>();
+    args.tile_rows = (!MERGED && a.tile_rows && (tile_bytes + slot_bytes + STB) * MINB <= CLASS_DYN_SMEM_MAX) ? 1 : 0;
     const size_t smem = (args.tile_rows ? tile_bytes : 0) + slot_bytes + STB;
     // the opt-in limit is raised to the per-CTA maximum, not to this launch's
     // size: a captured graph may hold a larger launch
@@ -1853,25 +1891,26 @@ cudaError_t launch_shape(const ClassArgs &a, cudaStream_t st) {
     // the rest of the SM's 256 KB stays L1 (the class's Rys table rows, pair
     // data and D): a shared-memory carveout of what MINB resident CTAs use
     {
-        const size_t need = smem * (size_t)MINB;
+        const size_t need = smem * (size_t)(MINB * (CLASS_THREADS / threads));
         const int carve = need == 0 ? 0 : (int)std::min<size_t>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024));
         static FuncAttrs attrs;
-        e = attrs.set((const void *)class_kernel<LA, LB, LC, LD, R, BATCH, V>, CLASS_DYN_SMEM_MAX, carve);
+        e = attrs.set((const void *)class_kernel<LA, LB, LC, LD, R, BATCH, MERGED, V>, CLASS_DYN_SMEM_MAX, carve);
         if (e != cudaSuccess) return e;
     }
-    class_kernel<LA, LB, LC, LD, R, BATCH, V><<<(unsigned)a.ntasks, CLASS_THREADS, smem, st>>>(args);
+    class_kernel<LA, LB, LC, LD, R, BATCH, MERGED, V><<<(unsigned)a.ntasks, threads, smem, st>>>(args);
     return cudaGetLastError();
 }
 
 template <int LA, int LB, int LC, int LD, typename R>
 cudaError_t launch_variant(const ClassArgs &a, int variant, cudaStream_t st) {
+    if (a.items) return launch_shape<LA, LB, LC, LD, R, false, true, 0>(a, st);  // merged tasks: the default shape
     if (variant == 1 && PassShape<LA, LB, LC, LD, R, 1>::DISTINCT) {
-        if constexpr (PassShape<LA, LB, LC, LD, R, 1>::DISTINCT) return launch_shape<LA, LB, LC, LD, R, false, 1>(a, st);
+        if constexpr (PassShape<LA, LB, LC, LD, R, 1>::DISTINCT) return launch_shape<LA, LB, LC, LD, R, false, false, 1>(a, st);
     }
     if (variant == 2 && PassShape<LA, LB, LC, LD, R, 2>::DISTINCT) {
-        if constexpr (PassShape<LA, LB, LC, LD, R, 2>::DISTINCT) return launch_shape<LA, LB, LC, LD, R, false, 2>(a, st);
+        if constexpr (PassShape<LA, LB, LC, LD, R, 2>::DISTINCT) return launch_shape<LA, LB, LC, LD, R, false, false, 2>(a, st);
     }
-    return launch_shape<LA, LB, LC, LD, R, false, 0>(a, st);
+    return launch_shape<LA, LB, LC, LD, R, false, false, 0>(a, st);
 }
 
 // precision 0: FP64, 1: FP32; variant: shape variant (0..NVARIANT-1; a
@@ -1880,8 +1919,8 @@ template <int LA, int LB, int LC, int LD>
 cudaError_t launch_t(const ClassArgs &a, int precision, int variant, cudaStream_t st) {
     if (a.ntasks <= 0) return cudaSuccess;
     if (a.mols) {
-        if (precision == 0) return launch_shape<LA, LB, LC, LD, double, true, 0>(a, st);
-        return launch_shape<LA, LB, LC, LD, float, true, 0>(a, st);
+        if (precision == 0) return launch_shape<LA, LB, LC, LD, double, true, true, 0>(a, st);
+        return launch_shape<LA, LB, LC, LD, float, true, true, 0>(a, st);
     }
     if (precision == 0) return launch_variant<LA, LB, LC, LD, double>(a, variant, st);
     return launch_variant<LA, LB, LC, LD, float>(a, variant, st);
