@@ -283,6 +283,11 @@ cudaError_t launch_class(int k, const LaunchCtx &ctx, const DevPlan &plan, const
 // f class k (NKERN <= k < NKALL), FP64: a group of warps evaluates and digests
 // each quartet of its task
 cudaError_t launch_fclass(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, int nbf);
+// small builds: the f classes of one CTA size in one launch (fclass_threads:
+// threads per quartet of class k, 32, 64, 128 or 256)
+int fclass_threads(int k);
+cudaError_t launch_fgroup(int threads, int n, const int *ks, const LaunchCtx &ctx, const DevPlan *plans,
+                          const RankSplit *rs, int nbf);
 // adds {count, sum, xor} of the hashes of the quartets a launch of class k over
 // this plan's task list would evaluate to out[0..2] (zeroed by the caller)
 // (fp32: the list of a mixed build's FP32 kets)

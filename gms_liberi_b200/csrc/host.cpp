@@ -653,6 +653,8 @@ static void balance_items(const PairsHost &pr, int k, int rank, int nsize, PlanH
 // lanes per quartet are the fewest that bring a quartet below half the even
 // spread, but not below UNIT_FLOOR_US, where a warp's own start and digestion
 // dominate.
+// Builds of at most so many f quartets launch their f classes grouped by CTA size.
+static const long long FGROUP_MAX_QUARTETS = 60000;
 static const double UNIT_LANES = 148 * 16 * 32, UNIT_FLOOR_US = 5.0, UNIT_TAIL_US = 25.0;
 
 static void plan_units(const PairsHost &pr, PlanHost *plans) {
@@ -1244,7 +1246,28 @@ static int build_on_device(liberi_handle h, const double *dD, double *dF, cudaSt
     // f classes (FP64 in every precision mode), in the driver's order
     if (h->pairs.nl[3] > 0) {
         ctx.rys_tab7 = h->d_tab7;
-        for (int k = NKERN; k < NKALL; k++) {
+        long long nf = 0;
+        for (int k = NKERN; k < NKALL; k++) nf += h->fq[k - NKERN];
+        const bool grouped = fan && nf <= FGROUP_MAX_QUARTETS;
+        for (int gt = 256; gt >= 32 && grouped; gt /= 2) {
+            int ks[NKERN_F], n = 0;
+            DevPlan dps[NKERN_F];
+            RankSplit rss[NKERN_F];
+            for (int k = NKERN; k < NKALL; k++) {
+                if (h->plan[k].total == 0 || fclass_threads(k) != gt) continue;
+                ks[n] = k;
+                rss[n] = rank_split_of(h, k);
+                dps[n++] = dev_plan_of(h, k);
+            }
+            if (n == 0) continue;
+            int rc = fan_stream(&ctx.stream);
+            if (rc) return rc;
+            for (int s = 0; s < nspin; s++) {
+                set_spin(s);
+                CUDA_TRY(launch_fgroup(gt, n, ks, ctx, dps, rss, b.num_bas));
+            }
+        }
+        for (int k = NKERN; k < NKALL && !grouped; k++) {
             PlanHost &ph = h->plan[k];
             if (ph.total == 0) continue;
             DevPlan dp = dev_plan_of(h, k);

@@ -330,12 +330,13 @@ __device__ __forceinline__ void fdigest(double (&acc)[S::NCS][S::ND], bool rowok
 
 }  // namespace
 
-// SWAP: the class's ket pair holds the f shell and gives the rows.
+// Task `task` of a group (CTA or warp).  SWAP: the class's ket pair holds the f
+// shell and gives the rows.
 template <typename S, bool SWAP>
-__global__ void __launch_bounds__(S::BLOCK, S::MINB) fclass_kernel(ClassArgs a, const double *__restrict__ tab7) {
+__device__ __forceinline__ void fclass_task(const ClassArgs &a, const double *__restrict__ tab7, int block) {
     constexpr int GT = S::GT, NROW = S::NROW;
     const int grp = S::GROUPS > 1 ? (int)(threadIdx.x >> 5) : 0;
-    const int task = (int)blockIdx.x * S::GROUPS + grp;
+    const int task = block * S::GROUPS + grp;
     if (task >= a.ntasks) return;  // the whole group (only warp barriers follow where a CTA holds several)
     extern __shared__ __align__(16) double fsm[];
     double *sm = fsm + (size_t)grp * S::SMEM;
@@ -420,6 +421,55 @@ __global__ void __launch_bounds__(S::BLOCK, S::MINB) fclass_kernel(ClassArgs a, 
         }
         if (t.z > 1) group_sync<GT>();
     }
+}
+
+template <typename S, bool SWAP>
+__global__ void __launch_bounds__(S::BLOCK, S::MINB) fclass_kernel(const __grid_constant__ ClassArgs a,
+                                                                   const double *__restrict__ tab7) {
+    fclass_task<S, SWAP>(a, tab7, (int)blockIdx.x);
+}
+
+// shape of a class by its engine orientation: the rows are the bra pair where
+// that holds an f shell, else the ket pair
+template <int LA, int LB, int LC, int LD>
+struct FShape {
+    static constexpr bool SWAP = LA < 3;
+    static_assert(SWAP ? LC == 3 : LB >= LD || LC < 3, "rows: the larger f pair");
+    using S = typename std::conditional<SWAP, FR<LD, LA, LB>, FR<LB, LC, LD>>::type;
+};
+#define LIBERI_FCLASSES(X)                                                                                          \
+    X(21, 3, 3, 3, 3) X(22, 0, 0, 3, 0) X(23, 0, 0, 3, 1) X(24, 0, 0, 3, 2) X(25, 1, 0, 3, 0) X(26, 3, 3, 3, 0)         \
+    X(27, 3, 0, 1, 1) X(28, 3, 0, 2, 0) X(29, 2, 1, 3, 0) X(30, 2, 2, 3, 0) X(31, 3, 0, 3, 0) X(32, 3, 1, 1, 0)         \
+    X(33, 3, 1, 1, 1) X(34, 3, 1, 2, 0) X(35, 3, 1, 2, 1) X(36, 2, 2, 3, 1) X(37, 3, 1, 3, 0) X(38, 3, 1, 3, 1)         \
+    X(39, 3, 2, 1, 0) X(40, 3, 3, 3, 1) X(41, 3, 2, 1, 1) X(42, 3, 2, 2, 0) X(43, 3, 2, 2, 1) X(44, 3, 2, 2, 2)         \
+    X(45, 3, 2, 3, 0) X(46, 3, 2, 3, 1) X(47, 3, 2, 3, 2) X(48, 3, 3, 0, 0) X(49, 3, 3, 1, 0) X(50, 3, 3, 1, 1)         \
+    X(51, 3, 3, 2, 0) X(52, 3, 3, 2, 1) X(53, 3, 3, 2, 2) X(54, 3, 3, 3, 2)
+
+// Small builds: all classes of one CTA size (128 threads of warp groups, or
+// one group of 64, 128 or 256) in one launch; 34 launches of a few quartets
+// each were mostly launch time.
+struct FGroup {
+    const double *tab7;
+    int n;
+    int k[NKERN_F], first_block[NKERN_F];
+    ClassArgs a[NKERN_F];
+};
+template <typename S, bool SWAP>
+__device__ __noinline__ void fgroup_task(const ClassArgs &a, const double *tab7, int block) {
+    fclass_task<S, SWAP>(a, tab7, block);
+}
+template <int GT>
+__global__ void __launch_bounds__(GT == 32 ? 128 : GT) fgroup_kernel(const __grid_constant__ FGroup g) {
+    int c = 0;
+    while (c + 1 < g.n && (int)blockIdx.x >= g.first_block[c + 1]) c++;
+    const int block = (int)blockIdx.x - g.first_block[c];
+#define LIBERI_F(kk, A, B, C, D)                                                                     \
+    case kk:                                                                                        \
+        if constexpr (FShape<A, B, C, D>::S::GT == GT)                                               \
+            fgroup_task<typename FShape<A, B, C, D>::S, FShape<A, B, C, D>::SWAP>(g.a[c], g.tab7, block); \
+        break;
+    switch (g.k[c]) { LIBERI_FCLASSES(LIBERI_F) }
+#undef LIBERI_F
 }
 
 // Schwarz values of f pairs: one group per pair P of one class, the diagonal
@@ -516,13 +566,11 @@ cudaError_t launch_fschwarz(int pair_class, int npairs, int pair_off, const DevB
     }
 }
 
-// one class by its engine orientation (la lb lc ld): the rows are the bra pair
-// where that holds an f shell, else the ket pair
+// one class
 template <int LA, int LB, int LC, int LD>
 static cudaError_t fclass_t(const ClassArgs &a, const double *tab7, cudaStream_t stream) {
-    constexpr bool SWAP = LA < 3;
-    static_assert(SWAP ? LC == 3 : LB >= LD || LC < 3, "rows: the larger f pair");
-    using S = typename std::conditional<SWAP, FR<LD, LA, LB>, FR<LB, LC, LD>>::type;
+    using S = typename FShape<LA, LB, LC, LD>::S;
+    constexpr bool SWAP = FShape<LA, LB, LC, LD>::SWAP;
     const size_t smem = (size_t)S::GROUPS * S::SMEM * sizeof(double);
     static FuncAttrs attrs;
     cudaError_t e = attrs.set((const void *)fclass_kernel<S, SWAP>, (int)smem, -1);
@@ -532,8 +580,7 @@ static cudaError_t fclass_t(const ClassArgs &a, const double *tab7, cudaStream_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_fclass(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, int nbf) {
-    if (plan.ntasks <= 0) return cudaSuccess;
+static ClassArgs fclass_args(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, int nbf) {
     const KernelDesc &kd = KDESC[k];
     ClassArgs a{};
     a.b = ctx.basis;
@@ -543,7 +590,6 @@ cudaError_t launch_fclass(int k, const LaunchCtx &ctx, const DevPlan &plan, cons
     a.thr = kd.asym;
     a.strict = !kd.rys;
     a.tasks = plan.tasks;
-    a.ntasks_dev = nullptr;
     a.ntasks = plan.ntasks;
     a.nbf = nbf;
     a.bra_ids = plan.bra_ids;
@@ -554,22 +600,78 @@ cudaError_t launch_fclass(int k, const LaunchCtx &ctx, const DevPlan &plan, cons
     a.swapped = plan.swapped;
     a.rs = rs;
     a.k_offset = ctx.k_offset;
-    // the engine orientation (la lb lc ld) of classes 21..54, KDESC order
+    return a;
+}
+
+cudaError_t launch_fclass(int k, const LaunchCtx &ctx, const DevPlan &plan, const RankSplit &rs, int nbf) {
+    if (plan.ntasks <= 0) return cudaSuccess;
+    const ClassArgs a = fclass_args(k, ctx, plan, rs, nbf);
 #define LIBERI_F(kk, A, B, C, D) \
     case kk: return fclass_t<A, B, C, D>(a, ctx.rys_tab7, ctx.stream);
     switch (k) {
-        LIBERI_F(21, 3, 3, 3, 3) LIBERI_F(22, 0, 0, 3, 0) LIBERI_F(23, 0, 0, 3, 1) LIBERI_F(24, 0, 0, 3, 2)
-        LIBERI_F(25, 1, 0, 3, 0) LIBERI_F(26, 3, 3, 3, 0) LIBERI_F(27, 3, 0, 1, 1) LIBERI_F(28, 3, 0, 2, 0)
-        LIBERI_F(29, 2, 1, 3, 0) LIBERI_F(30, 2, 2, 3, 0) LIBERI_F(31, 3, 0, 3, 0) LIBERI_F(32, 3, 1, 1, 0)
-        LIBERI_F(33, 3, 1, 1, 1) LIBERI_F(34, 3, 1, 2, 0) LIBERI_F(35, 3, 1, 2, 1) LIBERI_F(36, 2, 2, 3, 1)
-        LIBERI_F(37, 3, 1, 3, 0) LIBERI_F(38, 3, 1, 3, 1) LIBERI_F(39, 3, 2, 1, 0) LIBERI_F(40, 3, 3, 3, 1)
-        LIBERI_F(41, 3, 2, 1, 1) LIBERI_F(42, 3, 2, 2, 0) LIBERI_F(43, 3, 2, 2, 1) LIBERI_F(44, 3, 2, 2, 2)
-        LIBERI_F(45, 3, 2, 3, 0) LIBERI_F(46, 3, 2, 3, 1) LIBERI_F(47, 3, 2, 3, 2) LIBERI_F(48, 3, 3, 0, 0)
-        LIBERI_F(49, 3, 3, 1, 0) LIBERI_F(50, 3, 3, 1, 1) LIBERI_F(51, 3, 3, 2, 0) LIBERI_F(52, 3, 3, 2, 1)
-        LIBERI_F(53, 3, 3, 2, 2) LIBERI_F(54, 3, 3, 3, 2)
+        LIBERI_FCLASSES(LIBERI_F)
         default: return cudaErrorInvalidValue;
     }
 #undef LIBERI_F
+}
+
+// CTA size, groups per CTA and shared bytes of class k
+static void fclass_shape(int k, int &gt, int &groups, size_t &smem) {
+#define LIBERI_F(kk, A, B, C, D)                                                      \
+    case kk:                                                                         \
+        gt = FShape<A, B, C, D>::S::GT;                                               \
+        groups = FShape<A, B, C, D>::S::GROUPS;                                       \
+        smem = sizeof(double) * (size_t)groups * FShape<A, B, C, D>::S::SMEM;         \
+        break;
+    switch (k) {
+        LIBERI_FCLASSES(LIBERI_F)
+        default: gt = 0; groups = 1; smem = 0;
+    }
+#undef LIBERI_F
+}
+
+template <int GT>
+static cudaError_t fgroup_t(const FGroup &g, int blocks, size_t smem, cudaStream_t stream) {
+    static FuncAttrs attrs;
+    cudaError_t e = attrs.set((const void *)fgroup_kernel<GT>, 96 * 1024, -1);  // above every class's need
+    if (e != cudaSuccess) return e;
+    fgroup_kernel<GT><<<(unsigned)blocks, GT == 32 ? 128 : GT, smem, stream>>>(g);
+    return cudaGetLastError();
+}
+
+int fclass_threads(int k) {
+    int gt, groups;
+    size_t bytes;
+    fclass_shape(k, gt, groups, bytes);
+    return gt;
+}
+
+cudaError_t launch_fgroup(int gt, int n, const int *ks, const LaunchCtx &ctx, const DevPlan *plans,
+                          const RankSplit *rs, int nbf) {
+    FGroup g{};
+    g.tab7 = ctx.rys_tab7;
+    int blocks = 0;
+    size_t smem = 0;
+    for (int i = 0; i < n; i++) {
+        int t, groups;
+        size_t bytes;
+        fclass_shape(ks[i], t, groups, bytes);
+        if (t != gt) return cudaErrorInvalidValue;
+        if (plans[i].ntasks <= 0) continue;
+        g.k[g.n] = ks[i];
+        g.first_block[g.n] = blocks;
+        g.a[g.n++] = fclass_args(ks[i], ctx, plans[i], rs[i], nbf);
+        blocks += (plans[i].ntasks + groups - 1) / groups;
+        smem = bytes > smem ? bytes : smem;
+    }
+    if (blocks == 0) return cudaSuccess;
+    switch (gt) {
+        case 32: return fgroup_t<32>(g, blocks, smem, ctx.stream);
+        case 64: return fgroup_t<64>(g, blocks, smem, ctx.stream);
+        case 128: return fgroup_t<128>(g, blocks, smem, ctx.stream);
+        case 256: return fgroup_t<256>(g, blocks, smem, ctx.stream);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace liberi
