@@ -242,6 +242,7 @@ struct DeviceBuffers {
     // matrices, and their float copies
     double *uhf_sq = nullptr;
     float *uhf_sqf = nullptr;
+    double *uhf_df = nullptr;  // host-buffer open-shell builds: the beta D and F
     long long *scratch_total = nullptr;  // device counters (mixed split)
     size_t bytes = 0;
 };

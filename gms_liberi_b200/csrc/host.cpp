@@ -216,6 +216,7 @@ struct liberi_handle_s {
     bool last_split_lists = false;  // the last build ran the per-build FP64/FP32 task lists
     bool last_units = false;        // ... and warp tasks for the classes planned so
     cudaEvent_t ev[NKERN + 1][2] = {};
+    cudaEvent_t build_ev[2] = {};  // around a host-buffer build (stats.build_ms)
     bool ev_recorded[NKERN] = {};
     bool plan_dirty = false;
 
@@ -1453,6 +1454,55 @@ static int batch_enqueue(liberi_batch b, cudaStream_t st, uint32_t mask) {
     return LIBERI_OK;
 }
 
+// Workspaces of the shell Schwarz generator: a stream and a device buffer that
+// starts with the Rys table.  A call takes the idle one of its device, or makes
+// its own when another thread has it, and leaves at most one per device, of at
+// most SZ_KEEP bytes; the last handle's destruction releases them.  Making and
+// releasing stream, buffer and table on each call took 0.6 of its 0.8 ms.
+struct SchwarzSpace {
+    cudaStream_t stream = nullptr;
+    unsigned char *buf = nullptr;
+    size_t cap = 0;
+};
+static const size_t SZ_KEEP = 8u << 20;
+static const int SZ_DEVICES = 64;
+static std::mutex g_sz_mu;
+static SchwarzSpace *g_sz[SZ_DEVICES] = {};
+static std::atomic<long long> g_live_handles{0};
+
+static void sz_destroy(SchwarzSpace *w) {
+    if (!w) return;
+    if (w->buf) cudaFreeAsync(w->buf, w->stream);
+    if (w->stream) cudaStreamDestroy(w->stream);
+    delete w;
+}
+// buffer of at least `bytes` after the table
+static cudaError_t sz_reserve(SchwarzSpace *w, size_t tab_bytes, size_t bytes) {
+    if (!w->stream) {
+        const cudaError_t e = high_priority_stream(&w->stream);
+        if (e != cudaSuccess) return e;
+    }
+    if (w->cap >= tab_bytes + bytes) return cudaSuccess;
+    if (w->buf) cudaFreeAsync(w->buf, w->stream);
+    w->buf = nullptr;
+    w->cap = 0;
+    const size_t cap = tab_bytes + std::max<size_t>(2 * bytes, 256 * 1024);
+    cudaError_t e = cudaMallocAsync((void **)&w->buf, cap, w->stream);
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpyAsync(w->buf, rys_table_host().data(), RYS_TABLE_SIZE * sizeof(double), cudaMemcpyHostToDevice, w->stream);
+    if (e == cudaSuccess) w->cap = cap;
+    return e;
+}
+static void sz_release_all() {
+    std::lock_guard<std::mutex> lk(g_sz_mu);
+    for (int d = 0; d < SZ_DEVICES; d++)
+        if (g_sz[d]) {
+            DeviceGuard guard(d);
+            sz_destroy(g_sz[d]);
+            g_sz[d] = nullptr;
+        }
+}
+
 // ================================ C ABI ===========================================
 extern "C" {
 
@@ -1548,6 +1598,7 @@ int liberi_c_create(liberi_handle *handle) {
     *handle = new (std::nothrow) liberi_handle_s();
     if (!*handle) return fail(LIBERI_E_NOMEM, "liberi_create: out of host memory");
     memset(&(*handle)->stats, 0, sizeof(liberi_stats));
+    g_live_handles++;
     return LIBERI_OK;
 }
 
@@ -1561,6 +1612,10 @@ int liberi_c_cleanup(liberi_handle h) {
                 cudaEventDestroy(h->ev[k][j]);
                 h->ev[k][j] = nullptr;
             }
+    for (cudaEvent_t &e : h->build_ev) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
     free_device(h);
     h->basis = BasisHost();
     h->pairs = PairsHost();
@@ -1572,6 +1627,7 @@ int liberi_c_destroy(liberi_handle h) {
     if (!h) return fail(LIBERI_E_ARG, "liberi_destroy: null handle");
     liberi_c_cleanup(h);
     delete h;
+    if (--g_live_handles == 0) sz_release_all();
     return LIBERI_OK;
 }
 
@@ -1632,9 +1688,7 @@ int liberi_c_setup(liberi_handle h, int32_t nsh, int32_t natoms, int32_t num_bas
     }
     DeviceGuard dev_guard(h->device);
     CUDA_TRY(dev_guard.err);
-    cudaDeviceProp prop;
-    CUDA_TRY(cudaGetDeviceProperties(&prop, h->device));
-    h->num_sms = prop.multiProcessorCount;
+    CUDA_TRY(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device));
     h->basis = std::move(b);
     h->my_rank = my_rank;
     h->num_procs = num_procs;
@@ -1697,17 +1751,20 @@ int liberi_c_fock_build_uhf(liberi_handle h, const double *density_a, const doub
     CUDA_TRY(dev_guard.err);
     cudaStream_t st = h->stream;
     const size_t bytes = (size_t)matrix_size * sizeof(double);
-    // the beta density and Fock matrix in a stream-ordered scratch pair beside the handle's own D and F
-    double *db = nullptr, *fb = nullptr;
-    CUDA_TRY(cudaMallocAsync((void **)&db, 2 * bytes, st));
-    fb = db + matrix_size;
+    // the beta density and Fock matrix beside the handle's own D and F, kept
+    // from the first open-shell call (allocating and releasing them on each
+    // cost 0.3 ms and more: the pool returns its memory at every synchronisation)
+    if (!h->dev.uhf_df) {
+        CUDA_TRY(cudaMallocAsync((void **)&h->dev.uhf_df, 2 * bytes, st));
+        h->allocs.push_back(h->dev.uhf_df);
+    }
+    double *db = h->dev.uhf_df, *fb = db + matrix_size;
     cudaError_t e = cudaMemcpyAsync(h->dev.D, density_a, bytes, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(db, density_b, bytes, cudaMemcpyHostToDevice, st);
     int rc = LIBERI_OK;
     if (e == cudaSuccess) rc = build_on_device(h, h->dev.D, h->dev.F, st, db, fb);
     if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(fock_a, h->dev.F, bytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(fock_b, fb, bytes, cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(db, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (rc) return rc;
     CUDA_TRY(e);
@@ -1725,25 +1782,19 @@ int liberi_c_fock_build(liberi_handle h, const double *density, double *fock, in
     DeviceGuard dev_guard(h->device);
     CUDA_TRY(dev_guard.err);
     cudaStream_t st = h->stream;
-    cudaEvent_t e0, e1;
-    CUDA_TRY(cudaEventCreate(&e0));
-    CUDA_TRY(cudaEventCreate(&e1));
+    for (cudaEvent_t &e : h->build_ev)
+        if (!e) CUDA_TRY(cudaEventCreate(&e));
+    const cudaEvent_t e0 = h->build_ev[0], e1 = h->build_ev[1];
     CUDA_TRY(cudaEventRecord(e0, st));
     CUDA_TRY(cudaMemcpyAsync(h->dev.D, density, (size_t)matrix_size * sizeof(double), cudaMemcpyHostToDevice, st));
     int rc = build_on_device(h, h->dev.D, h->dev.F, st);
-    if (rc) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        return rc;
-    }
+    if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(fock, h->dev.F, (size_t)matrix_size * sizeof(double), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaEventRecord(e1, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     h->stats.build_ms = ms;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     return LIBERI_OK;
 }
 
@@ -2257,17 +2308,14 @@ int liberi_c_quartet_fingerprint(liberi_handle h, uint64_t *out) { return quarte
 
 int liberi_c_quartet_fingerprint_all(liberi_handle h, uint64_t *out) { return quartet_fingerprint(h, NKALL, out); }
 
-// The table of an s/p/d basis from its shells: one allocation, one upload, one
-// launch, the packed table back.
-static int schwarz_shells(liberi_handle h, double *out) {
-    const BasisHost &b = h->basis;
-    const std::vector<double> &tab = rys_table_host();
+// The table of an s/p/d basis from its shells: one upload, one launch, the
+// packed table back.
+static int schwarz_shells(const BasisHost &b, int device, double *out) {
     // (exponents and coefficients shell by shell: an s and a p shell may name the same sh_loc)
     const size_t nsh = (size_t)b.nsh, ntri = nsh * (nsh + 1) / 2;
     const size_t nex = (size_t)std::accumulate(b.contr_num.begin(), b.contr_num.end(), 0LL);
     const size_t o_xyz = dev_round(nsh * sizeof(int4)), o_ex = o_xyz + dev_round(nsh * sizeof(double4));
-    const size_t o_co = o_ex + dev_round(nex * sizeof(double)), o_tab = o_co + dev_round(nex * sizeof(double));
-    const size_t o_out = o_tab + dev_round(tab.size() * sizeof(double));
+    const size_t o_co = o_ex + dev_round(nex * sizeof(double)), o_out = o_co + dev_round(nex * sizeof(double));
     std::vector<unsigned char> host(o_out);
     int4 *shell = reinterpret_cast<int4 *>(host.data());
     double4 *xyz = reinterpret_cast<double4 *>(host.data() + o_xyz);
@@ -2283,16 +2331,32 @@ static int schwarz_shells(liberi_handle h, double *out) {
         std::copy(c.begin() + lo, c.begin() + lo + b.contr_num[s], co + at);
         at += b.contr_num[s];
     }
-    std::memcpy(host.data() + o_tab, tab.data(), tab.size() * sizeof(double));
-    unsigned char *d = nullptr;
-    CUDA_TRY(cudaMallocAsync((void **)&d, o_out + ntri * sizeof(double), h->stream));
-    h->allocs.push_back(d);
-    CUDA_TRY(cudaMemcpyAsync(d, host.data(), o_out, cudaMemcpyHostToDevice, h->stream));
-    const ShellTable t{(const int4 *)d, (const double4 *)(d + o_xyz), (const double *)(d + o_ex),
-                       (const double *)(d + o_co), (const double *)(d + o_tab), CUX, SQRT_TWOPI52};
-    CUDA_TRY(launch_schwarz_shells(t, b.nsh, (double *)(d + o_out), h->stream));
-    CUDA_TRY(cudaMemcpyAsync(out, d + o_out, ntri * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    SchwarzSpace *w = nullptr;
+    if (device < SZ_DEVICES) {
+        std::lock_guard<std::mutex> lk(g_sz_mu);
+        std::swap(w, g_sz[device]);
+    }
+    if (!w) w = new (std::nothrow) SchwarzSpace();
+    if (!w) return fail(LIBERI_E_NOMEM, "liberi_schwarz: out of host memory");
+    const size_t tab_bytes = dev_round(RYS_TABLE_SIZE * sizeof(double));
+    cudaError_t e = sz_reserve(w, tab_bytes, o_out + ntri * sizeof(double));
+    if (e == cudaSuccess) {
+        unsigned char *d = w->buf + tab_bytes;
+        e = cudaMemcpyAsync(d, host.data(), o_out, cudaMemcpyHostToDevice, w->stream);
+        const ShellTable t{(const int4 *)d, (const double4 *)(d + o_xyz), (const double *)(d + o_ex),
+                           (const double *)(d + o_co), (const double *)w->buf, CUX, SQRT_TWOPI52};
+        if (e == cudaSuccess) e = launch_schwarz_shells(t, b.nsh, (double *)(d + o_out), w->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(out, d + o_out, ntri * sizeof(double), cudaMemcpyDeviceToHost, w->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(w->stream);
+    }
+    if (e == cudaSuccess && w->cap <= SZ_KEEP && device < SZ_DEVICES) {
+        std::lock_guard<std::mutex> lk(g_sz_mu);
+        std::swap(w, g_sz[device]);  // (another thread's workspace left meanwhile goes instead)
+    }
+    sz_destroy(w);
+    if (e == cudaErrorMemoryAllocation) return fail(LIBERI_E_NOMEM, "liberi_schwarz: %s", cudaGetErrorString(e));
+    CUDA_TRY(e);
     return LIBERI_OK;
 }
 
@@ -2311,12 +2375,9 @@ int liberi_c_schwarz(int32_t nsh, int32_t natoms, int32_t num_bas, int32_t mxgto
     rc = validate_basis(tmp.basis);
     if (rc) return rc;
     CUDA_TRY(cudaGetDevice(&tmp.device));  // the caller's current device
+    if (std::find(tmp.basis.ang_mom.begin(), tmp.basis.ang_mom.end(), 4) == tmp.basis.ang_mom.end())
+        return schwarz_shells(tmp.basis, tmp.device, schwrz_out);
     CUDA_TRY(high_priority_stream(&tmp.stream));
-    if (std::find(tmp.basis.ang_mom.begin(), tmp.basis.ang_mom.end(), 4) == tmp.basis.ang_mom.end()) {
-        rc = schwarz_shells(&tmp, schwrz_out);
-        free_device(&tmp);
-        return rc;
-    }
     // f shells: the f classes' evaluation reads pair arrays
     std::vector<double4> shell_xyz;
     build_pairs(tmp.basis, tmp.pairs, shell_xyz);
