@@ -47,7 +47,13 @@ constexpr int BOYS_ROW = 2 * RYS_NCOEF;
 __host__ __device__ constexpr int boys_off(int m) {
     return rys_herm_off(MAXROOT + 1) + (RYS_NCOEF - rys_herm_off(MAXROOT + 1) % RYS_NCOEF) + (m - 1) * BOYS_NINT * BOYS_ROW;
 }
-constexpr int RYS_TABLE_SIZE = boys_off(BOYS_MMAX + 1);
+// m = 1 alone (the largest class, (ps|ss)): intervals of width 1/16, F_0 at the
+// middle and the degree-6 coefficients of F_1; F_0 follows by integration, so a
+// row is eight doubles where F_1 and exp(-T) take sixteen.
+constexpr int BOYS1_PER_UNIT = 16;
+constexpr int BOYS1_NINT = 25 * BOYS1_PER_UNIT + 1;
+constexpr int BOYS1_OFF = boys_off(BOYS_MMAX + 1);
+constexpr int RYS_TABLE_SIZE = BOYS1_OFF + BOYS1_NINT * RYS_NCOEF;
 // Single-precision tables for the FP32 tier: intervals of width 1/8 on
 // [0, RYS_TMAX), degree-3 power basis in x = 2(8T - k) - 1 (4 coefficients:
 // two functions per 256-bit load; interpolation error below 5e-8 relative);

@@ -162,6 +162,21 @@ __device__ __forceinline__ void boys_eval(double T, const double *__restrict__ t
         for (int m = 1; m <= M; m++) F[m] = F[m - 1] * ((m - 0.5) * it);
         return;
     }
+    if constexpr (M == 1) {
+        const double t = T * (double)BOYS1_PER_UNIT;
+        const int k = (int)t;
+        const double x = 2.0 * (t - (double)k) - 1.0, x2 = x * x, x4 = x2 * x2;
+        double f0, c0, c1, c2, c3, c4, c5, c6;
+        const double *b = tab + BOYS1_OFF + (size_t)k * RYS_NCOEF;
+        ldg_v4f64(b, f0, c0, c1, c2);
+        ldg_v4f64(b + 4, c3, c4, c5, c6);
+        F[1] = fma(fma(c6, x2, fma(c5, x, c4)), x4, fma(fma(c3, x, c2), x2, fma(c1, x, c0)));
+        // F_0(x) = F_0(0) - (1/32) sum c_i x^(i+1) / (i+1)
+        const double s = fma(fma(c6 * (1.0 / 7), x2, fma(c5 * (1.0 / 6), x, c4 * 0.2)), x4,
+                             fma(fma(c3 * 0.25, x, c2 * (1.0 / 3)), x2, fma(c1 * 0.5, x, c0)));
+        F[0] = fma(x * (-0.5 / BOYS1_PER_UNIT), s, f0);
+        return;
+    }
     const double t8 = T * (double)BOYS_PER_UNIT;
     const int k = (int)t8;
     const double x = 2.0 * (t8 - (double)k) - 1.0, x2 = x * x, x4 = x2 * x2;

@@ -276,10 +276,24 @@ void fill_table(int nmax, int nint, OffT tab_off, HermT herm_off, std::vector<do
     }
 }
 
+void fill_boys1(std::vector<double> &out) {
+    const int M = RYS_NCOEF - 1;
+    for (int k = 0; k < BOYS1_NINT; k++) {
+        std::vector<double> f(M);
+        for (int i = 0; i < M; i++)
+            f[i] = (double)boys_series(1, (k + 0.5L * (std::cos(PI * (i + 0.5) / M) + 1.0L)) / BOYS1_PER_UNIT);
+        const std::vector<double> pf = cheb_to_power(f);
+        double *dst = &out[BOYS1_OFF + (size_t)k * RYS_NCOEF];
+        dst[0] = (double)boys_series(0, (k + 0.5L) / BOYS1_PER_UNIT);
+        for (int i = 0; i < M; i++) dst[1 + i] = pf[i];
+    }
+}
+
 void build_tables() {
     g_table.assign(RYS_TABLE_SIZE, 0.0);
     fill_table(MAXROOT, RYS_NINT, rys_table_off, rys_herm_off, g_table);
     fill_boys(RYS_NCOEF, boys_off, g_table);
+    fill_boys1(g_table);
 }
 
 std::vector<double> g_table7;
