@@ -53,7 +53,12 @@ __host__ __device__ constexpr int boys_off(int m) {
 constexpr int BOYS1_PER_UNIT = 16;
 constexpr int BOYS1_NINT = 25 * BOYS1_PER_UNIT + 1;
 constexpr int BOYS1_OFF = boys_off(BOYS_MMAX + 1);
-constexpr int RYS_TABLE_SIZE = BOYS1_OFF + BOYS1_NINT * RYS_NCOEF;
+// m = 2: intervals of width 1/32, F_0 and F_1 at the middle and the degree-5
+// coefficients of F_2, integrated once and twice.
+constexpr int BOYS2_PER_UNIT = 32;
+constexpr int BOYS2_NINT = 25 * BOYS2_PER_UNIT + 1;
+constexpr int BOYS2_OFF = BOYS1_OFF + BOYS1_NINT * RYS_NCOEF;
+constexpr int RYS_TABLE_SIZE = BOYS2_OFF + BOYS2_NINT * RYS_NCOEF;
 // Single-precision tables for the FP32 tier: intervals of width 1/8 on
 // [0, RYS_TMAX), degree-3 power basis in x = 2(8T - k) - 1 (4 coefficients:
 // two functions per 256-bit load; interpolation error below 5e-8 relative);

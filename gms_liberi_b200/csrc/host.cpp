@@ -473,7 +473,9 @@ static void by_cost(CostedTasks &lst, std::vector<int4> &out) {
 // Merged tasks of class k: a row's concatenated items (t.x = item0 + the row's
 // first) cut where a warp has task_us of work (MERGE_TASK_US in one-warp CTAs,
 // so that a task of uncontracted kets pays for its start), at most `cap` kets.
-static const double MERGE_TASK_US = 60.0;
+// (Longer in batches, whose tasks outnumber the resident warps many times: 40
+// molecules 44.0 ms at 60 us, 43.0 at 150; a 40-atom molecule alone 3.30 and 3.35.)
+static const double MERGE_TASK_US = 60.0, MERGE_BATCH_US = 150.0;
 static void merged_tasks(const PairsHost &pr, const PlanHost &ph, int k, int cap, double task_us, int item0,
                          CostedTasks &out) {
     for (const int2 &r : ph.rows) {
@@ -1380,7 +1382,7 @@ static int batch_build_tasks(liberi_batch b, int k) {
     CostedTasks lst;
     int item0 = 0;
     for (liberi_handle h : b->hs) {
-        merged_tasks(h->pairs, h->plan[k], k, b->chunk[k], MERGE_TASK_US, item0, lst);
+        merged_tasks(h->pairs, h->plan[k], k, b->chunk[k], MERGE_BATCH_US, item0, lst);
         item0 += (int)h->plan[k].items.size();
     }
     by_cost(lst, tasks);

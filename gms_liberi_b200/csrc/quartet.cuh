@@ -150,9 +150,11 @@ __device__ __forceinline__ void rys_eval_staged(double T, double thr, bool stric
     }
 }
 // ---- Boys functions of the Obara-Saika classes ----------------------------------
-// F_0..F_M(T) for the classes with the large-T form above T = 25: one row of
-// F_M and exp(-T) (four 256-bit loads; the two roots and weights of the Rys
-// rule take eight) and the downward recursion, whose terms are all positive.
+// F_0..F_M(T) for the classes with the large-T form above T = 25.  One table row:
+// for M <= 2 eight doubles (two 256-bit loads), F_M as a polynomial and the lower
+// orders by integrating it from their values at the interval's middle; for
+// M > 2 F_M and exp(-T) (four loads) and the downward recursion, whose terms
+// are all positive.  The two roots and weights of the Rys rule take eight loads.
 template <int M>
 __device__ __forceinline__ void boys_eval(double T, const double *__restrict__ tab, double (&F)[M + 1]) {
     if (T > 25.0) {
@@ -175,6 +177,24 @@ __device__ __forceinline__ void boys_eval(double T, const double *__restrict__ t
         const double s = fma(fma(c6 * (1.0 / 7), x2, fma(c5 * (1.0 / 6), x, c4 * 0.2)), x4,
                              fma(fma(c3 * 0.25, x, c2 * (1.0 / 3)), x2, fma(c1 * 0.5, x, c0)));
         F[0] = fma(x * (-0.5 / BOYS1_PER_UNIT), s, f0);
+        return;
+    }
+    if constexpr (M == 2) {
+        const double t = T * (double)BOYS2_PER_UNIT;
+        const int k = (int)t;
+        const double x = 2.0 * (t - (double)k) - 1.0, x2 = x * x, x4 = x2 * x2;
+        const double d = x * (-0.5 / BOYS2_PER_UNIT);  // minus the distance from the middle
+        double f0, f1, c0, c1, c2, c3, c4, c5;
+        const double *b = tab + BOYS2_OFF + (size_t)k * RYS_NCOEF;
+        ldg_v4f64(b, f0, f1, c0, c1);
+        ldg_v4f64(b + 4, c2, c3, c4, c5);
+        F[2] = fma(fma(c5, x, c4), x4, fma(fma(c3, x, c2), x2, fma(c1, x, c0)));
+        const double s1 = fma(fma(c5 * (1.0 / 6), x, c4 * 0.2), x4,
+                              fma(fma(c3 * 0.25, x, c2 * (1.0 / 3)), x2, fma(c1 * 0.5, x, c0)));
+        // (the term of c5 in the second integral is below 1e-17)
+        const double s2 = fma(c4 * (1.0 / 30), x4, fma(fma(c3 * 0.05, x, c2 * (1.0 / 12)), x2, fma(c1 * (1.0 / 6), x, c0 * 0.5)));
+        F[1] = fma(d, s1, f1);
+        F[0] = fma(d, fma(d, s2, f1), f0);
         return;
     }
     const double t8 = T * (double)BOYS_PER_UNIT;
@@ -221,10 +241,11 @@ __device__ __forceinline__ void boys_eval(float T, const float *__restrict__ tab
 // total angular momentum 1..3.  About half the FP64 operations of the Rys
 // form (one row and the recurrences once a primitive quartet, not once a
 // root) and half its table loads or fewer.  Measured on C60 in FP64:
-// (sp|sp) 13.17 -> 11.33 ms, (sp|pp) 13.28 -> 11.83, (sp|pd) 9.93 -> 8.81,
-// (ss|pp) 6.07 -> 5.09, (sp|sd) 4.30 -> 3.92, (ss|pd) 2.91 -> 2.61,
-// (ss|sd) 1.86 -> 1.62, (ss|sp) 10.89 -> 10.82; the build 103.5 -> 97.2 ms.
-// (On Rys roots as moments the recurrences alone had gained nothing.)
+// (sp|sp) 13.17 -> 10.64 ms, (sp|pp) 13.28 -> 11.82, (ss|sp) 10.89 -> 9.28,
+// (sp|pd) 9.93 -> 8.81, (ss|pp) 6.07 -> 4.65, (sp|sd) 4.30 -> 3.92, (ss|pd)
+// 2.91 -> 2.61, (ss|sd) 1.86 -> 1.56; the build 103.5 -> 94.4 ms.  (On Rys
+// roots as moments the recurrences alone had gained nothing, and with rows of
+// sixteen doubles (ss|sp) 10.82 and (sp|sp) 11.36: the gathers bound them.)
 constexpr bool os_key(int key) {
     return key == 1000 || key == 1010 || key == 1100 || key == 1110 || key == 2000 || key == 2010 || key == 2100 ||
            key == 2110;

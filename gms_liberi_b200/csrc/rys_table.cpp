@@ -289,11 +289,26 @@ void fill_boys1(std::vector<double> &out) {
     }
 }
 
+void fill_boys2(std::vector<double> &out) {
+    const int M = RYS_NCOEF - 2;
+    for (int k = 0; k < BOYS2_NINT; k++) {
+        std::vector<double> f(M);
+        for (int i = 0; i < M; i++)
+            f[i] = (double)boys_series(2, (k + 0.5L * (std::cos(PI * (i + 0.5) / M) + 1.0L)) / BOYS2_PER_UNIT);
+        const std::vector<double> pf = cheb_to_power(f);
+        double *dst = &out[BOYS2_OFF + (size_t)k * RYS_NCOEF];
+        dst[0] = (double)boys_series(0, (k + 0.5L) / BOYS2_PER_UNIT);
+        dst[1] = (double)boys_series(1, (k + 0.5L) / BOYS2_PER_UNIT);
+        for (int i = 0; i < M; i++) dst[2 + i] = pf[i];
+    }
+}
+
 void build_tables() {
     g_table.assign(RYS_TABLE_SIZE, 0.0);
     fill_table(MAXROOT, RYS_NINT, rys_table_off, rys_herm_off, g_table);
     fill_boys(RYS_NCOEF, boys_off, g_table);
     fill_boys1(g_table);
+    fill_boys2(g_table);
 }
 
 std::vector<double> g_table7;
