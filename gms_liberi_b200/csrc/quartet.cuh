@@ -237,18 +237,18 @@ __device__ __forceinline__ void boys_eval(float T, const float *__restrict__ tab
 }
 
 // Classes evaluated by the Obara-Saika recurrences on Boys functions.
-// The single-pass classes with at most one p function beside a shell pair of
-// total angular momentum 1..3.  About half the FP64 operations of the Rys
-// form (one row and the recurrences once a primitive quartet, not once a
-// root) and half its table loads or fewer.  Measured on C60 in FP64:
-// (sp|sp) 13.17 -> 10.64 ms, (sp|pp) 13.28 -> 11.82, (ss|sp) 10.89 -> 9.28,
-// (sp|pd) 9.93 -> 8.81, (ss|pp) 6.07 -> 4.65, (sp|sd) 4.30 -> 3.92, (ss|pd)
-// 2.91 -> 2.61, (ss|sd) 1.86 -> 1.56; the build 103.5 -> 94.4 ms.  (On Rys
-// roots as moments the recurrences alone had gained nothing, and with rows of
-// sixteen doubles (ss|sp) 10.82 and (sp|sp) 11.36: the gathers bound them.)
+// The single-pass classes of total angular momentum 1..4 with an s second ket
+// shell, (dd|ss) aside.  About half the FP64 operations of the Rys form (one row
+// and the recurrences once a primitive quartet, not once a root) and half its
+// table loads or fewer.  Measured on C60 in FP64: (sp|sp) 13.17 -> 10.64 ms,
+// (sp|pp) 13.28 -> 11.82, (ss|sp) 10.89 -> 9.28, (sp|pd) 9.93 -> 8.81, (ss|pp)
+// 6.07 -> 4.65, (sp|sd) 4.30 -> 3.92, (pp|sd) 3.75 -> 3.68, (ss|pd) 2.91 -> 2.61,
+// (ss|sd) 1.86 -> 1.56, (sd|sd) 0.60 -> 0.56; the build 103.5 -> 94.3 ms.  (On
+// Rys roots as moments the recurrences alone had gained nothing, and with rows
+// of sixteen doubles (ss|sp) took 10.82 and (sp|sp) 11.36: the gathers bound them.)
 constexpr bool os_key(int key) {
     return key == 1000 || key == 1010 || key == 1100 || key == 1110 || key == 2000 || key == 2010 || key == 2100 ||
-           key == 2110;
+           key == 2110 || key == 1120 || key == 2020;
 }
 template <int LA, int LB, int LC, int LD>
 constexpr bool os_class() {
@@ -762,7 +762,8 @@ __device__ __forceinline__ void contract_hgp_pair(const F2 (&gx)[LA + LB + 1][LC
 // J. Chem. Phys. 84 (1986) 3963): c[m] = F_m times the prefactors; pa = P-A,
 // qc = Q-C, wp = W-P, wq = W-Q, hp = 1/2p, rp = q/(p+q), h = 1/2(p+q).
 // add(e, ic, x, y) adds x*y to (e0|c0), e over the functions of angular
-// momentum LA..LA+LB, ic over those of C (LC <= 1).
+// momentum LA..LA+LB, ic over those of C (LC <= 2; hq = 1/2q and rq = p/(p+q)
+// for LC = 2).
 __host__ __device__ constexpr int cart_exp(int l, int i, int ax) {
     return ax == 0 ? cart_x(l, i) : (ax == 1 ? cart_y(l, i) : cart_z(l, i));
 }
@@ -777,9 +778,8 @@ __host__ __device__ constexpr int lower_pos(int l, int i, int ax, int k) {
     return cart_pos(l - k, cart_x(l, i) - (ax == 0 ? k : 0), cart_y(l, i) - (ax == 1 ? k : 0));
 }
 template <int LA, int LB, int LC, typename R, typename Add>
-__device__ __forceinline__ void os_add(const R (&c)[LA + LB + LC + 1], const R (&pa)[3],
-                                       const R (&qc)[3], const R (&wp)[3], const R (&wq)[3], R hp,
-                                       R rp, R h, Add add) {
+__device__ __forceinline__ void os_add(const R (&c)[LA + LB + LC + 1], const R (&pa)[3], const R (&qc)[3],
+                                       const R (&wp)[3], const R (&wq)[3], R hp, R rp, R h, R hq, R rq, Add add) {
     constexpr int L = LA + LB, M = L + LC;
     R v[L + 1][M + 1][ncart(L)];  // (a s|s s)^(m), a of angular momentum l: m <= M - l
 #pragma unroll
@@ -800,17 +800,42 @@ __device__ __forceinline__ void os_add(const R (&c)[LA + LB + LC + 1], const R (
                 }
                 v[l][m][e] = t;
             }
+    // (e s|l s)^(m) of one function e and a p function l of C
+    auto ket = [&](int le, int e, int m, int l) {
+        R t = fma(wq[l], v[le][m + 1][e], qc[l] * v[le][m][e]);
+        const int n = cart_exp(le, e, l);
+        if (n > 0) t = fma(R(n) * h, v[le > 0 ? le - 1 : 0][m + 1][n > 0 ? lower_pos(le, e, l, 1) : 0], t);
+        return t;
+    };
 #pragma unroll
     for (int e = 0; e < nrange(LA, L); e++) {
         const int le = range_l(LA, e), ie = range_i(LA, e);
         if constexpr (LC == 0) add(e, 0, v[le][0][ie], R(1));
-        else {
+        else if constexpr (LC == 1) {
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 add(e, k, qc[k], v[le][0][ie]);
                 add(e, k, wq[k], v[le][1][ie]);
                 const int n = cart_exp(le, ie, k);
                 if (n > 0) add(e, k, R(n) * h, v[le - 1][1][lower_pos(le, ie, k, 1)]);
+            }
+        } else {
+            // d functions of C: axis x raised on |l), pairs 00 11 22 01 02 12
+            const int X[6] = {0, 1, 2, 1, 2, 2}, Y[6] = {0, 1, 2, 0, 0, 1};
+            R k0[3], k1[3];
+#pragma unroll
+            for (int l = 0; l < 3; l++) {
+                k0[l] = ket(le, ie, 0, l);
+                k1[l] = ket(le, ie, 1, l);
+            }
+            const R t = fma(-rq, v[le][1][ie], v[le][0][ie]);
+#pragma unroll
+            for (int f = 0; f < 6; f++) {
+                const int x = X[f], l = Y[f], n = cart_exp(le, ie, x);
+                add(e, f, qc[x], k0[l]);
+                add(e, f, wq[x], k1[l]);
+                if (x == l) add(e, f, hq, t);
+                if (n > 0) add(e, f, R(n) * h, ket(le - 1, n > 0 ? lower_pos(le, ie, x, 1) : 0, 1, l));
             }
         }
     }
@@ -882,7 +907,7 @@ __device__ __forceinline__ void eval_block(const DevBasis &b, int p0, int np, in
                     const double qc[3] = {Qp.x - C.x, Qp.y - C.y, Qp.z - C.z};
                     const double wp[3] = {-rq * pqx, -rq * pqy, -rq * pqz};
                     const double wq[3] = {rpp * pqx, rpp * pqy, rpp * pqz};
-                    os_add<LA, LB, LC>(c, pa, qc, wp, wq, hp, rq, 0.5 * ipq, [&](int e, int ic, R x, R y) {
+                    os_add<LA, LB, LC>(c, pa, qc, wp, wq, hp, rq, 0.5 * ipq, hq, rpp, [&](int e, int ic, R x, R y) {
                         if constexpr (HGP) acc[e][ic] = fma(x, y, acc[e][ic]);
                         else acc[e][0][ic][0] = fma(x, y, acc[e][0][ic][0]);
                     });
@@ -970,7 +995,7 @@ __device__ __forceinline__ void eval_block(const DevBasis &b, int p0, int np, in
                     for (int m = 0; m <= M; m++) c[m] *= pref;
                     const float pa[3] = {Pa.x, Pa.y, Pa.z}, qc[3] = {Qa.x, Qa.y, Qa.z};
                     const float wp[3] = {-rq * pqx, -rq * pqy, -rq * pqz}, wq[3] = {rpp * pqx, rpp * pqy, rpp * pqz};
-                    os_add<LA, LB, LC>(c, pa, qc, wp, wq, hp, rq, 0.5f * ipq, [&](int e, int ic, R x, R y) {
+                    os_add<LA, LB, LC>(c, pa, qc, wp, wq, hp, rq, 0.5f * ipq, hq, rpp, [&](int e, int ic, R x, R y) {
                         if constexpr (HGP) acc[e][ic] = fma(x, y, acc[e][ic]);
                         else acc[e][0][ic][0] = fma(x, y, acc[e][0][ic][0]);
                     });
@@ -1107,10 +1132,9 @@ __device__ __forceinline__ T dget(const T *__restrict__ Dm, unsigned ld, unsigne
 // register allocator.  The table was tuned offline with ptxas register and
 // spill reports; LIBERI_TUNE_* override one class for that search.  The FP64
 // resident-CTA counts were measured again, per class, on C60 with the
-// shared-memory carveout sized to the resident CTAs and the staged table
-// rows (every count from three below to one above the earlier choice):
-// (sp|sp) 6 -> 4 (14.10 -> 12.99 ms: no spills, and its table rows out of
-// L1), (sp|sd) 5 -> 4 (4.96 -> 4.14), (ss|sd) 6 -> 5 (1.91 -> 1.75), (sd|sd)
+// shared-memory carveout sized to the resident CTAs (every count from three
+// below to one above the earlier choice): (sp|sp) 6 -> 4 (14.10 -> 12.99 ms,
+// no spills), (sp|sd) 5 -> 4 (4.96 -> 4.14), (ss|sd) 6 -> 5 (1.91 -> 1.75), (sd|sd)
 // 2 -> 3 (0.73 -> 0.70), (dd|dd) 2 -> 1 (0.45 -> 0.33 ms).
 constexpr int class_key(int la, int lb, int lc, int ld) { return la * 1000 + lb * 100 + lc * 10 + ld; }
 constexpr int tuned_nmu(int key) {
