@@ -284,6 +284,21 @@ __device__ __forceinline__ void digest_unit(const R (&acc)[NMU][NBU][ncart(LC)][
         }
 }
 
+// Obara-Saika contribution of one primitive quartet to (e0|c0) (os_add): c the
+// Boys values, hp = 1/2p, pq = P-Q, pa = P-A, qc = Q-C.
+template <int LA, int LB, int LC, typename R>
+__device__ __forceinline__ void unit_os(R (&c)[LA + LB + LC + 1], R pref, R p, R q, R ipq, R hp, R pqx, R pqy, R pqz,
+                                        R pax, R pay, R paz, R qcx, R qcy, R qcz,
+                                        R (&acc)[nrange(LA, LA + LB)][ncart(LC)][1]) {
+    const R rq = q * ipq, rp = p * ipq;
+#pragma unroll
+    for (int m = 0; m <= LA + LB + LC; m++) c[m] *= pref;
+    const R pa[3] = {pax, pay, paz}, qc[3] = {qcx, qcy, qcz};
+    const R wp[3] = {-rq * pqx, -rq * pqy, -rq * pqz}, wq[3] = {rp * pqx, rp * pqy, rp * pqz};
+    os_add<LA, LB, LC>(c, pa, qc, wp, wq, hp, rq, R(0.5) * ipq, R(0), rp,  // (LC <= 1 here)
+                       [&](int e, int ic, R x, R y) { acc[e][ic][0] = fma(x, y, acc[e][ic][0]); });
+}
+
 // One warp task: row pair t.x against kets t.y .. t.y+t.z-1, t.z * PG <= 32.
 template <int LA, int LB, int LC, int LD, typename R, int NS>
 __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, int4 t) {
@@ -322,24 +337,28 @@ __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, in
     const unsigned long long kpr = (unsigned long long)__double_as_longlong(r1.w);
     const int q0 = (int)(unsigned)kpr, nprim = act ? np * (int)(unsigned)(kpr >> 32) : 0;
 
+    // The Obara-Saika classes sum (e0|c0) (contract as in quartet.cuh, no roots
+    // to share out), the others the (ab|cd) block of this pass.
+    constexpr bool OS = os_class<LA, LB, LC, LD>() && NMU == S::NA && NBU == S::NB;
+    constexpr int NE = OS ? nrange(LA, LAB) : NMU * NBU;
+    R acc[NE][NC][ND];
+#pragma unroll
+    for (int e = 0; e < NE; e++)
+#pragma unroll
+        for (int ic = 0; ic < NC; ic++)
+#pragma unroll
+            for (int id = 0; id < ND; id++) acc[e][ic][id] = R(0);
     int ex[NMU], ey[NMU], ez[NMU];
-    R acc[NMU][NBU][NC][ND];
 #pragma unroll
     for (int m = 0; m < NMU; m++) {
         ex[m] = cx_rt(LA, mu0 + m);
         ey[m] = cy_rt(LA, mu0 + m);
         ez[m] = cz_rt(LA, mu0 + m);
-#pragma unroll
-        for (int n = 0; n < NBU; n++)
-#pragma unroll
-            for (int ic = 0; ic < NC; ic++)
-#pragma unroll
-                for (int id = 0; id < ND; id++) acc[m][n][ic][id] = R(0);
     }
     // the quartet's UG lanes: over its primitive quartets first, over the
     // roots where there are more lanes than primitive quartets
     int up = UG;
-    while (up > 1 && up > nprim) up >>= 1;
+    while (!OS && up > 1 && up > nprim) up >>= 1;
     const int ur = UG / up;
 #pragma unroll 1
     for (int i = usub & (up - 1); i < nprim; i += up) {
@@ -352,6 +371,12 @@ __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, in
             const double rs = rsqrt(p + q), ipq = rs * rs;
             const double T = p * q * ipq * (pqx * pqx + pqy * pqy + pqz * pqz);
             const double pref = Px.x * Qx.x * rs;
+            if constexpr (OS) {
+                double c[LAB + LCD + 1];
+                boys_eval<LAB + LCD>(T, a.tab, c);
+                unit_os<LA, LB, LC>(c, pref, p, q, ipq, hp, pqx, pqy, pqz, Pp.x - A.x, Pp.y - A.y, Pp.z - A.z,
+                                    Qp.x - C.x, Qp.y - C.y, Qp.z - C.z, acc);
+            } else {
 #pragma unroll 1
             for (int r = usub / up; r < NR; r += ur) {
                 double ui, wr;
@@ -364,8 +389,9 @@ __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, in
                 vrr<LAB, LCD, double>(gx, (Pp.x - A.x) - fq * pqx, (Qp.x - C.x) + fp * pqx, b10, b01, b00, 1.0);
                 vrr<LAB, LCD, double>(gy, (Pp.y - A.y) - fq * pqy, (Qp.y - C.y) + fp * pqy, b10, b01, b00, 1.0);
                 vrr<LAB, LCD, double>(gz, (Pp.z - A.z) - fq * pqz, (Qp.z - C.z) + fp * pqz, b10, b01, b00, wr);
-                contract_unit<LA, LB, LC, LD, double, NMU, NBU>(gx, gy, gz, abx, aby, abz, cdx, cdy, cdz, ex, ey, ez,
-                                                                nu0, acc);
+                contract_unit<LA, LB, LC, LD, double, NMU, NBU>(gx, gy, gz, abx, aby, abz, cdx, cdy, cdz, ex, ey, ez, nu0,
+                                                                reinterpret_cast<double(&)[NMU][NBU][NC][ND]>(acc));
+            }
             }
         } else {
             // primitive screening of the FP32 tier (eval_block)
@@ -383,6 +409,11 @@ __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, in
             const float rs = rsqrtf(p + q), ipq = rs * rs;
             const float T = p * q * ipq * (pqx * pqx + pqy * pqy + pqz * pqz);
             const float pref = Pa.w * Qa.w * rs;
+            if constexpr (OS) {
+                float c[LAB + LCD + 1];
+                boys_eval<LAB + LCD>(T, a.tabf, c);
+                unit_os<LA, LB, LC>(c, pref, p, q, ipq, hp, pqx, pqy, pqz, Pa.x, Pa.y, Pa.z, Qa.x, Qa.y, Qa.z, acc);
+            } else {
 #pragma unroll 1
             for (int r = usub / up; r < NR; r += ur) {
                 float ui, wr;
@@ -395,8 +426,9 @@ __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, in
                 vrr<LAB, LCD, float>(gx, Pa.x - fq * pqx, Qa.x + fp * pqx, b10, b01, b00, 1.0f);
                 vrr<LAB, LCD, float>(gy, Pa.y - fq * pqy, Qa.y + fp * pqy, b10, b01, b00, 1.0f);
                 vrr<LAB, LCD, float>(gz, Pa.z - fq * pqz, Qa.z + fp * pqz, b10, b01, b00, wr);
-                contract_unit<LA, LB, LC, LD, float, NMU, NBU>(gx, gy, gz, abx, aby, abz, cdx, cdy, cdz, ex, ey, ez,
-                                                               nu0, acc);
+                contract_unit<LA, LB, LC, LD, float, NMU, NBU>(gx, gy, gz, abx, aby, abz, cdx, cdy, cdz, ex, ey, ez, nu0,
+                                                               reinterpret_cast<float(&)[NMU][NBU][NC][ND]>(acc));
+            }
             }
         }
     }
@@ -404,14 +436,26 @@ __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, in
 #pragma unroll 1
     for (int o = PG; o < PG * UG; o <<= 1) {
 #pragma unroll
-        for (int m = 0; m < NMU; m++)
+        for (int e = 0; e < NE; e++)
 #pragma unroll
-            for (int n = 0; n < NBU; n++)
+            for (int ic = 0; ic < NC; ic++)
 #pragma unroll
-                for (int ic = 0; ic < NC; ic++)
+                for (int id = 0; id < ND; id++) acc[e][ic][id] += __shfl_xor_sync(0xffffffffu, acc[e][ic][id], o);
+    }
+    R blk[NMU][NBU][NC][ND];
 #pragma unroll
-                    for (int id = 0; id < ND; id++)
-                        acc[m][n][ic][id] += __shfl_xor_sync(0xffffffffu, acc[m][n][ic][id], o);
+    for (int m = 0; m < NMU; m++) {
+        R sl[NBU][NC][1];
+        if constexpr (OS && LB > 0) bra_transfer<LA, LB, LC, R>(reinterpret_cast<R(&)[NE][NC]>(acc), m, abx, aby, abz, sl);
+#pragma unroll
+        for (int n = 0; n < NBU; n++)
+#pragma unroll
+            for (int ic = 0; ic < NC; ic++)
+#pragma unroll
+                for (int id = 0; id < ND; id++) {
+                    if constexpr (OS && LB > 0) blk[m][n][ic][id] = sl[n][ic][0];
+                    else blk[m][n][ic][id] = acc[m * NBU + n][ic][id];
+                }
     }
     QuartetCtx<R> qc;
     qc.bfA = b.shell_bf0[sab.x];
@@ -434,7 +478,7 @@ __device__ __noinline__ void unit_task(const UnitArgs &a, const UnitClass &u, in
     double *F[NS];
     F[0] = a.F;
     if constexpr (NS > 1) F[1] = a.F2;
-    if (act && usub == 0) digest_unit<LA, LB, LC, LD, R, NMU, NBU, NS>(acc, mu0, nu0, qc, a.k_offset, F, jab);
+    if (act && usub == 0) digest_unit<LA, LB, LC, LD, R, NMU, NBU, NS>(blk, mu0, nu0, qc, a.k_offset, F, jab);
     __syncwarp();
     // the row pair's J: lanes of equal psub hold the same components
 #pragma unroll
