@@ -8,20 +8,22 @@
 // surviving ket pairs Q = (C, D) (the kets of a bra form a prefix of the
 // Schwarz-sorted ket list).  Each thread evaluates whole quartets:
 //   1. loop over kept primitive pairs (ket outer, bra inner, as the reference
-//      does, e.g. int0001.F90:220-287), evaluate Rys roots and weights from
-//      the piecewise tables, build 2D integrals with the vertical and
-//      horizontal recurrences in registers and contract the Cartesian block;
-//      large classes run the primitive loop in register-bounded passes over
-//      the components of shell A;
+//      does, e.g. int0001.F90:220-287): the low-L classes of os_key by the
+//      Obara-Saika recurrences on tabulated Boys functions, the others with
+//      Rys roots and weights from the piecewise tables, 2D integrals by the
+//      vertical and horizontal recurrences in registers and the contracted
+//      Cartesian block, large classes in register-bounded passes over the
+//      components of shell A;
 //   2. digest with the reference's DIRFCK rules (unique components for
 //      identical shells, 0.5 factors, skip |v| < cut, the six updates of
 //      int0000.F90:241-311 / int2222_rysgen.F90:11176-11338), pre-reduced in
 //      registers per quartet:
-//        K updates into rows A and B of F -> shared-memory tile of the CTA
+//        K updates into rows A and B of F -> FP64 global atomics (or, option
+//                                            tile_mask, a shared-memory tile
+//                                            flushed when the CTA ends)
 //        J update of the row pair (A,B)   -> summed over the warp (shuffles),
-//                                            one tile update per warp
+//                                            one update per warp
 //        J update of the ket pair (C,D)   -> FP64 global atomics
-//      and the tile is flushed to F with FP64 atomics when the CTA ends.
 // The FP32 instantiation evaluates step 1 entirely in single precision (pair
 // data rounded once from FP64, Rys roots and weights from single-precision
 // tables, recurrences and contraction) for the quartets whose Schwarz bound
